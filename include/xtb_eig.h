@@ -79,7 +79,7 @@ int xtb_dsygvd_device(int n, double* a, int lda, double* b, int ldb, double* w, 
  * device memory, for callers that cannot let a library allocate device memory (they manage every byte on the GPU
  * through their own pool or allocator, and a cudaMalloc/cudaFree inside a library call would break their budget
  * and may synchronise the device).  The call allocates nothing: its scratch is a static device array of about
- * 57 KB that the library holds on every GPU it is loaded on.  Limits: 1 <= n <= XTB_NOALLOC_MAX_N (larger n
+ * 173 KB that the library holds on every GPU it is loaded on.  Limits: 1 <= n <= XTB_NOALLOC_MAX_N (larger n
  * returns -1), lda >= n (else -3), and the device must hold the resident rows in shared memory (else -4; B200 does
  * for every n up to the maximum).  Every call looks up the array's device address; the first lookup on a device may
  * load the library's device code there, so make the first call before any stream capture.  Calls share the array:
@@ -221,8 +221,8 @@ int xtb_dsygvd_density_adjoint_batched(int count, const int* n, const double* co
  * "batch_grid" (1, default: inside the batch calls, each problem's resident reduction takes the fewest CTAs that
  * hold its rows in shared memory, so that problems run side by side; the results are bit for bit those of single
  * solves; 0 = the single-solve grid),
- * "test_barrier_stall" (failure-detection test hook, default 0; 1: the resident reduction's grid barriers wait for one
- * CTA more than the grid has, so every wait runs into "wait_limit_ms" and the call returns the barrier-timeout status
+ * "test_barrier_stall" (failure-detection test hook, default 0; 1: every exchange of the resident reduction also waits
+ * for a value that no CTA publishes, so the wait runs into "wait_limit_ms" and the call returns the barrier-timeout status
  * -2001 (info) or 1 (xtb_gpu_last_status) instead of hanging; host-pointer calls only, never for production use).
  * Returns 0, -1 for an unknown name, or -2 for a value out of range. */
 int xtb_gpu_set_option(const char* name, long value);

@@ -345,6 +345,9 @@ uint64_t wait_limit_ns() { return (uint64_t)g_wait_ms.load() * 1000000ull; }
 
 // ------------------------------------------------------------------------------------------------ stages
 
+// Slots per third of the reduction's exchange ring: a fence per this many columns, 3 x 16 n bytes (FP64) for each.
+constexpr int kSytrdRing = 32;
+
 template <typename T>
 void stage_sytrd(Call& k, int n, const T* dfull, int ldf, T* dout, int lda, T* d, T* e, T* tau) {
   if (!k.ok() || n <= 0) return;
@@ -371,11 +374,9 @@ void stage_sytrd(Call& k, int n, const T* dfull, int ldf, T* dout, int lda, T* d
   p.d = d;
   p.e = e;
   p.tau = tau;
-  T* xch = k.template dev<T>("sytrd.xch", 4 * (size_t)n);
-  unsigned* ctr = k.template dev<unsigned>("sytrd.ctr", 64);
+  p.ring_h = kSytrdRing;
+  p.xch = k.template dev<T>("sytrd.xch", sytrd_ring_elems(n, p.ring_h));
   if (!k.ok()) return;
-  p.xch = xch;
-  p.counter = ctr;
   p.st = k.c->d_status;
   p.rows_per_cta = pl.rows_per_cta;
   p.ldr = pl.ldr;
@@ -387,7 +388,7 @@ void stage_sytrd(Call& k, int n, const T* dfull, int ldf, T* dout, int lda, T* d
     if (!k.ok()) return;
   }
   // The last columns (all of them for a small matrix) on one CTA: the grid kernel hands the trailing block over.
-  // The failure-detection hook needs the grid barriers, so it keeps the grid kernel throughout.
+  // The failure-detection hook acts on the grid kernel's exchange, so it keeps that kernel throughout.
   const int tail = p.extra_members ? 0 : std::min(n, t_plan.tail);
   if (tail > 1 && tail == n) {
     k.check(sytrd_tail_launch<T>(p, 0, k.s), "sytrd tail launch");
@@ -399,8 +400,7 @@ void stage_sytrd(Call& k, int n, const T* dfull, int ldf, T* dout, int lda, T* d
     p.ldh = tail;
     if (!k.ok()) return;
   }
-  k.check(cudaMemsetAsync(ctr, 0, 64 * sizeof(unsigned), k.s), "sytrd counter");
-  if (k.ok()) k.check(sytrd_launch<T>(p, pl, k.s), "sytrd launch");
+  k.check(sytrd_launch<T>(p, pl, k.s), "sytrd launch");
   if (k.ok() && tail > 1) {
     SytrdParams<T> q = p;
     q.n = tail;

@@ -25,17 +25,18 @@ struct SytrdParams {
   T* d;
   T* e;
   T* tau;
-  T* xch;          // 2 x n (y_r, A(r,k-1)) pairs, two alternating exchange buffers
+  T* xch;          // exchange ring: 3 ring_h slots of n + 1 ((A x)_r, A(r,k-1)) pairs (sytrd_ring_elems values)
+  int ring_h;      // slots per third of the ring, >= 2
   T* grows;        // global row slab when rows do not fit shared memory (grid * rows_per_cta * ldr)
-  unsigned* counter;
+  unsigned* counter;  // in-place variant: its one grid barrier's counter (zero at launch)
   DeviceStatus* st;
   int rows_per_cta;
   int ldr;
   int use_smem;
   uint64_t limit_ns;
-  // Members the grid barriers wait for beyond the grid itself: 0 in every solve.  The library's failure-detection
-  // test hook (option "test_barrier_stall") sets 1, so that no barrier can complete and every wait runs into its
-  // time limit and returns an error status instead of hanging.
+  // 0 in every solve.  The library's failure-detection test hook (option "test_barrier_stall") sets 1: every
+  // exchange then also waits for a pair that no CTA publishes, so the wait runs into its time limit and the call
+  // returns an error status instead of hanging.
   int extra_members;
   // Grid kernel: k_stop > 0 hands the trailing (k_stop + 1) x (k_stop + 1) block over after step k_stop + 1 (that
   // step's update applied, full symmetric rows into hand, ld ldh) and returns; sytrd_tail_launch finishes it.
@@ -45,11 +46,19 @@ struct SytrdParams {
 };
 
 struct SytrdPlan {
-  int grid, threads, cpt, rows_per_cta, ldr;
+  int grid, threads, cpt, reg_rows, rows_per_cta, ldr;
   bool rows_in_smem, supported;
   size_t smem;
 };
 
+// Values of an exchange ring for matrices of order n: slots of n + 1 pairs (one for the failure-detection hook), a slot
+// a whole number of 32-byte sectors.
+__host__ __device__ inline size_t sytrd_ring_elems(int n, int ring_h) {
+  return (size_t)3 * ring_h * 2 * (((size_t)n + 4) & ~size_t(3));
+}
+// Rows are dealt to the CTAs in blocks whose pairs fill one 32-byte sector of the ring.
+template <typename T>
+__host__ __device__ constexpr int sytrd_row_block() { return 16 / (int)sizeof(T); }
 template <typename T>
 SytrdPlan sytrd_plan(int n, int num_sms, size_t max_smem, int grid_override);
 template <typename T>

@@ -3,7 +3,7 @@
 // allocator, a fixed per-process budget) and cannot allow a third-party call to cudaMalloc or cudaFree, which take
 // memory outside that budget and may synchronise the whole device.  This entry point therefore allocates nothing:
 // the caller passes the matrix and the outputs in device memory, and the kernel's scratch (barrier counter, device
-// status word and the two double-buffered exchange vectors) lives in the file-scope array below, which every GPU that
+// status word and the exchange ring) lives in the file-scope array below, which every GPU that
 // loads the library holds until the process exits.
 //
 // Host code may not use the array's name as a device address (on the host it names a stand-in object): every call
@@ -25,8 +25,9 @@ namespace {
 constexpr int kMaxN = XTB_NOALLOC_MAX_N;
 constexpr size_t kStatusOffset = 0;    // DeviceStatus
 constexpr size_t kCounterOffset = 256;  // 64 unsigned barrier counters
-constexpr size_t kVectorOffset = 512;   // y and next-column exchange vectors, 2 x 2 x kMaxN doubles
-constexpr size_t kScratchBytes = kVectorOffset + 4 * (size_t)kMaxN * sizeof(double);
+constexpr size_t kVectorOffset = 512;   // the exchange ring, 3 x kRing slots of kMaxN + 1 pairs
+constexpr int kRing = 2;                // the shortest ring: the array stays small
+constexpr size_t kScratchBytes = kVectorOffset + (size_t)3 * kRing * 2 * (kMaxN + 4) * sizeof(double);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -57,7 +58,7 @@ extern "C" int xtb_dsytrd_upper_noalloc(int n, double* a, int lda, double* d, do
   if (err == cudaSuccess) err = scratch_address(&base);
   if (err != cudaSuccess) return -1000 - (int)err;
   const SytrdPlan pl = sytrd_plan<double>(n, sms, (size_t)smem > 2048 ? (size_t)smem - 2048 : (size_t)smem, 0);
-  if (!pl.rows_in_smem || pl.threads != 512 || pl.cpt > 4) return -4;
+  if (!pl.rows_in_smem) return -4;
 
   SytrdParams<double> p{};
   p.n = n;
@@ -69,6 +70,7 @@ extern "C" int xtb_dsytrd_upper_noalloc(int n, double* a, int lda, double* d, do
   p.e = e;
   p.tau = tau;
   p.xch = reinterpret_cast<double*>(base + kVectorOffset);
+  p.ring_h = kRing;
   p.counter = reinterpret_cast<unsigned*>(base + kCounterOffset);
   p.st = reinterpret_cast<DeviceStatus*>(base + kStatusOffset);
   p.grows = nullptr;
@@ -76,7 +78,7 @@ extern "C" int xtb_dsytrd_upper_noalloc(int n, double* a, int lda, double* d, do
   p.ldr = pl.ldr;
   p.use_smem = 1;
   p.limit_ns = option_wait_limit_ns();
-  // Status word and barrier counter must start at zero; the exchange vectors are written before they are read.
+  // Status word and barrier counter must start at zero; the launch empties the exchange ring.
   err = cudaMemsetAsync(base, 0, kVectorOffset, s);
   if (err == cudaSuccess) err = sytrd_launch_upper_inplace(p, pl, s);
   DeviceStatus st{};

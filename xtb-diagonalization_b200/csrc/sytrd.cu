@@ -5,30 +5,47 @@
 //
 // B200 design (not a port of the reference's blocked CPU code).  The reduction is a chain of n-1 dependent
 // matrix-vector products, so on a GPU its cost is the grid-wide dependency per column, not flops.  One persistent
-// cooperative kernel keeps the whole symmetric matrix resident: CTA c of G owns rows c, c+G, c+2G, ... (cyclic, so
-// the shrinking trailing matrix stays balanced), in shared memory when they fit (n = 1788 FP64: 13 rows x 1788 x 8 B =
-// 186 KB per CTA on 148 SMs) and otherwise in a global (L2-resident) slab.  Per column k every CTA
-//   1. holds x = A(0:k-1, k) in registers (column c of the trailing matrix lives in thread c mod NT) and writes its
-//      warps' partial sums of ||x(0:k-2)||^2 to shared memory (no block-wide sync here);
+// cooperative kernel keeps the whole symmetric matrix on chip: rows are dealt to the CTAs in small blocks, cyclically
+// (so the shrinking trailing matrix stays balanced); a CTA's first RR rows live in registers (thread t holds the column
+// pairs 2(t + j NT), + 1 of them), the others in shared memory or, when they do not fit, in a global (L2-resident) slab.
+// Per column k every CTA
+//   1. holds x = A(0:k-1, k) in registers (the columns of thread t) and in shared memory;
 //   2. in ONE pass over its own rows applies the previous step's rank-2 update A -= v w^T + w v^T and accumulates
 //      (A x)_r with x itself rather than v: v = (scale x(0:k-2), 1), so y = A v = scale (A x)_r + A(r, k-1), and
-//      the Householder scalars are not needed before the pass (the update of step k+1 fused with the symv of step k;
-//      the per-row partial sums are combined by a reduce-scatter across the warp's lanes, 9 shuffles for 8 rows);
+//      the Householder scalars are not needed before the pass (the update of step k+1 fused with the symv of step k);
 //      the previous w at own rows is formed from the previous y and v at own rows, w = tau y - tau^2/2 (y.v) v, as
 //      the owner of each column forms it;
-//   3. after the pass's __syncthreads (which also publishes the ||x||^2 partials) publishes ((A x)_r, A(r,k-1)) for
-//      its rows and arrives at the grid barrier (a release-add on a counter); while the barrier is in flight it forms
-//      beta, tau, scale and v exactly as every other CTA does (same data, same summation order => bit-identical v in
-//      all CTAs), y at its own rows and its output columns; then it waits (an acquire poll, no further fences) and
-//      reads every row's pair for its columns, y = scale (A x) + A(:,k-1) with the owner's fma.  Two exchange buffers
-//      alternate: a CTA
-//      writes buffer p again only two steps later, after the barrier of the step in between, which every CTA reaches
-//      only after it has read buffer p.  (Polling per-value readiness flags instead of one counter was measured
-//      slower: 75k threads polling L2 cost more than one counter round trip.);
-//   4. forms w = tau y - tau^2/2 (y.v) v and the next x = A(0:k-2, k-1) - v w(k-1) - w v(k-1) redundantly.
-// One grid barrier and two block-level syncs per column; every reduction runs in a fixed order that does not depend
+//   3. after the pass's __syncthreads (which also publishes the ||x||^2 partials) one thread per own row publishes
+//      the pair ((A x)_r, A(r,k-1)) with one relaxed store, and every thread forms beta, tau, scale and v exactly as
+//      every other CTA does (same data, same summation order => bit-identical v in all CTAs);
+//   4. reads every row's pair for its columns.  There is no barrier: a slot of the exchange ring holds a NaN pattern
+//      no result can have until its pair arrives, and the reader polls the pair itself.  y = scale (A x) + A(:,k-1)
+//      with the owner's fma;
+//   5. forms w = tau y - tau^2/2 (y.v) v and the next x = A(0:k-2, k-1) - v w(k-1) - w v(k-1) redundantly.
+// Two block-level syncs and one L2 round trip per column; every reduction runs in a fixed order that does not depend
 // on the grid, so results are deterministic, identical across CTAs and the same for every grid size; every wait is
 // time-limited (device status word, no trap).
+//
+// What bounds it: latency.  An exchange of 1788 pairs among 148 CTAs alone takes 4700 cycles with an arrival counter
+// (store, fence, counter, poll, then the loads) and 2300 with polled pairs; of 412 pairs 3700 and 1900.  Two things make
+// the polled form work: neighbouring rows belong to one CTA, so that no two CTAs write one 32-byte sector (with cyclic
+// single rows, sectors shared by writers and polled meanwhile, the same exchange took 8000 cycles), and the first poll
+// comes only after the Householder scalars, about when the pairs arrive.  Inside the CTA, the rows were bound by
+// shared memory (every element loaded and stored each column: 186 KB twice per column and SM at n = 1788); 8 of 14 rows
+// in registers leave it 6.  Eight warps instead of sixteen halve the shuffles and the cross-warp sums, and a column's
+// code is specialised on the column pairs still active, so that it is straight-line and its dependent chains interleave.
+// Whole stage, FP64, before -> after: n = 1788 7.19 -> 4.52 ms (4.0 -> 2.5 us per column), 1203 4.27 -> 2.70,
+// 619 1.88 -> 1.21, 412 1.19 -> 0.69; FP32 n = 1788 6.24 -> 3.85.
+//
+// The ring has three thirds of H slots; step t uses slot t mod 3H.  In step t = bH + 1, after publishing, the owner
+// of a row puts the empty pattern back into its entries of third (b - 1) mod 3 and every thread executes a fence.
+// Every CTA has then read all of third (b - 1) mod 3 (it published step t - 1 = bH only after reading step bH - 1,
+// and this CTA has read its step bH).  The third is polled again from step (b + 2)H on; by then the reader has seen
+// a later publish of the same owner thread (step bH + 2 or later, H >= 2) and executed its own fence of step
+// (b + 1)H + 1, so the emptying happens before the poll.  A fence costs about 1000 cycles while stores are in flight,
+// so a third has 32 slots (8: 2 % slower).
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -38,7 +55,7 @@ namespace {
 
 constexpr int kRowChunk = 8;  // rows whose partial dot products are reduce-scattered together
 
-// Relaxed (morally strong) pair accesses of the exchange buffer (read after the grid barrier).
+// Relaxed (morally strong) accesses of the exchange ring: each value of a pair is its own 8- (4-)byte access.
 __device__ __forceinline__ void st_pair(double* p, double a, double b) {
   asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(a), "d"(b) : "memory");
 }
@@ -52,279 +69,506 @@ __device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
   asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p) : "memory");
 }
 
-// Block sum with a compile-time warp count: one __syncthreads; `scratch` (NW values) must not be reused by another
-// block_sum before every thread has passed this call's __syncthreads and read it (callers rotate scratch slots).
-template <int NW, typename T>
-__device__ __forceinline__ T block_sum_nw(T v, T* scratch) {
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-  __syncthreads();
-  T r = T(0);
+// The empty pattern is all ones (a NaN); a value whose high word is all ones counts as empty, so the publisher turns
+// such a NaN (only an input's payload can be one) into the default NaN.
+__device__ __forceinline__ bool is_empty(double x) { return __double2hiint(x) == -1; }
+__device__ __forceinline__ bool is_empty(float x) { return __float_as_int(x) == -1; }
+__device__ __forceinline__ double published(double x) {
+  return is_empty(x) ? __longlong_as_double(0x7ff8000000000000ll) : x;
+}
+__device__ __forceinline__ float published(float x) { return is_empty(x) ? __int_as_float(0x7fc00000) : x; }
+template <typename T>
+__device__ __forceinline__ T empty_value();
+template <>
+__device__ __forceinline__ double empty_value<double>() { return __longlong_as_double(-1ll); }
+template <>
+__device__ __forceinline__ float empty_value<float>() { return __int_as_float(-1); }
+
+template <typename T>
+struct __align__(2 * sizeof(T)) Pair {
+  T a, b;
+};
+
+// Sum of N values (N a power of two) read from shared memory, as a balanced tree: log2 N dependent additions.
+template <int N, typename T>
+__device__ __forceinline__ T tree_sum(const T* p, int stride) {
+  T v[N];
 #pragma unroll
-  for (int w = 0; w < NW; ++w) r += scratch[w];
-  return r;
+  for (int i = 0; i < N; ++i) v[i] = p[i * stride];
+#pragma unroll
+  for (int s = 1; s < N; s *= 2)
+#pragma unroll
+    for (int i = 0; i + s < N; i += 2 * s) v[i] += v[i + s];
+  return v[0];
 }
 
-// Reduce-scatter of 8 per-lane partial sums across the warp: on return lane l holds the warp-wide sum of row
-// (l >> 2) & 7 (complete in lanes with (l & 3) == 0).
-template <typename T>
-__device__ __forceinline__ T warp_reduce_scatter8(T (&acc)[kRowChunk]) {
+// FP64 matrix instruction D = A B (8 x 4 times 4 x 8; lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4)], + 1).
+// With A all ones, D[m][n] is the sum of B's column n, that is of the four lanes of quad n, for every m: a lane receives
+// the sums of quads 2(l%4) and 2(l%4) + 1.
+__device__ __forceinline__ void quad_sums(double v, double& even, double& odd) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+               : "=d"(even), "=d"(odd)
+               : "d"(1.0), "d"(v), "d"(0.0));
+}
+
+// Sum over the warp, in every lane: two matrix instructions (77 cycles) instead of five shuffles (191).
+__device__ __forceinline__ double warp_sum_mma(double v) {
+  double a, b;
+  quad_sums(v, a, b);
+  quad_sums(a + b, a, b);
+  return a;
+}
+__device__ __forceinline__ float warp_sum_mma(float v) { return warp_sum(v); }
+
+// The warp-wide sums of ROWS (8 or 4) per-lane values each to out[0 .. ROWS): halves are exchanged (added) across lanes
+// 16, 8 and 4, which leaves every row in one quad (in two), whose lanes one matrix instruction sums.  Both forms add in
+// the same order, so a row's sum does not depend on how many rows its CTA has.
+template <int ROWS>
+__device__ __forceinline__ void warp_row_sums(double (&acc)[kRowChunk], double* out) {
   const unsigned lane = threadIdx.x & 31;
   const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const T send = h4 ? acc[i] : acc[i + 4];
-    const T keep = h4 ? acc[i + 4] : acc[i];
+  for (int i = 0; i < ROWS / 2; ++i) {
+    const double send = h4 ? acc[i] : acc[i + ROWS / 2], keep = h4 ? acc[i + ROWS / 2] : acc[i];
     acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const T send = h3 ? acc[i] : acc[i + 2];
-    const T keep = h3 ? acc[i + 2] : acc[i];
+  for (int i = 0; i < ROWS / 4; ++i) {
+    const double send = h3 ? acc[i] : acc[i + ROWS / 4], keep = h3 ? acc[i + ROWS / 4] : acc[i];
     acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
   }
-  {
-    const T send = h2 ? acc[0] : acc[1];
-    const T keep = h2 ? acc[1] : acc[0];
-    acc[0] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  double even, odd;
+  if constexpr (ROWS == 8) {
+    const double send = h2 ? acc[0] : acc[1], keep = h2 ? acc[1] : acc[0];
+    quad_sums(keep + __shfl_xor_sync(0xffffffffu, send, 4), even, odd);
+    if (lane < 4) *reinterpret_cast<Pair<double>*>(out + 2 * lane) = Pair<double>{even, odd};
+  } else {
+    quad_sums(acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 4), even, odd);
+    if (lane < 4) out[lane] = even;  // row l is in quads 2l and 2l + 1
   }
-  T r = acc[0];
+}
+template <int ROWS>
+__device__ __forceinline__ void warp_row_sums(float (&acc)[kRowChunk], float* out) {
+  const unsigned lane = threadIdx.x & 31;
+  const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < ROWS / 2; ++i) {
+    const float send = h4 ? acc[i] : acc[i + ROWS / 2], keep = h4 ? acc[i + ROWS / 2] : acc[i];
+    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS / 4; ++i) {
+    const float send = h3 ? acc[i] : acc[i + ROWS / 4], keep = h3 ? acc[i + ROWS / 4] : acc[i];
+    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  float r = acc[0];
+  if constexpr (ROWS == 8) {
+    const float send = h2 ? acc[0] : acc[1], keep = h2 ? acc[1] : acc[0];
+    r = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  } else {
+    r += __shfl_xor_sync(0xffffffffu, r, 4);
+  }
   r += __shfl_xor_sync(0xffffffffu, r, 2);
   r += __shfl_xor_sync(0xffffffffu, r, 1);
-  return r;
+  if ((lane & 3) == 0 && (ROWS == 8 || h2 == false)) out[ROWS == 8 ? lane >> 2 : lane >> 3] = r;
+}
+
+// One row chunk of the pass over the first JA column pairs: ROWS register rows, or ROWS rows of shared (global) memory
+// with the last pair's columns tested against k.  Straight-line code, so that the rows' dependent chains interleave (a
+// branch per row and pair left every chain's latency exposed: 5700 cycles instead of 2000 for 13 rows of 1788).
+template <int ROWS, int JA, int CPT, typename T>
+__device__ __forceinline__ void pass_registers(T (*ra)[CPT], const Pair<T>* vy, T tau, T half, const T* wk, const T* vk,
+                                               const T* xs, T* acc) {
+  T vr[ROWS], wr[ROWS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const Pair<T> o = vy[q];
+    vr[q] = -o.a;
+    wr[q] = fma(-tau, o.b, half * o.a);  // -w, bit for bit the negative of the owner's w = tau y - half v
+  }
+#pragma unroll
+  for (int i = 0; i < 2 * JA; ++i) {
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      T a = fma(vr[q], wk[i], ra[q][i]);
+      a = fma(wr[q], vk[i], a);
+      ra[q][i] = a;
+      acc[q] = fma(a, xs[i], acc[q]);
+    }
+  }
+}
+
+template <int ROWS, int JA, int NT, typename T>
+__device__ __forceinline__ void pass_memory(T* row0, size_t ldr, int k, const Pair<T>* vy, T tau, T half, const T* wk,
+                                            const T* vk, const T* xs, T* acc) {
+  // Every load before the first store: the stores could alias the loads for all the compiler knows.
+  Pair<T> e[ROWS][JA];
+  const int c0 = 2 * (int)threadIdx.x;
+  const bool in = c0 + 2 * (JA - 1) * NT < k;  // the last pair's columns
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+    for (int j = 0; j < JA; ++j) {
+      if (j == JA - 1) e[q][j] = Pair<T>{T(0), T(0)};
+      if (j < JA - 1 || in) e[q][j] = *reinterpret_cast<const Pair<T>*>(row0 + q * ldr + c0 + 2 * j * NT);
+    }
+  T vr[ROWS], wr[ROWS];
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q) {
+    const Pair<T> o = vy[q];
+    vr[q] = -o.a;
+    wr[q] = fma(-tau, o.b, half * o.a);
+  }
+#pragma unroll
+  for (int j = 0; j < JA; ++j)
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      e[q][j].a = fma(wr[q], vk[2 * j], fma(vr[q], wk[2 * j], e[q][j].a));
+      e[q][j].b = fma(wr[q], vk[2 * j + 1], fma(vr[q], wk[2 * j + 1], e[q][j].b));
+      acc[q] = fma(e[q][j].b, xs[2 * j + 1], fma(e[q][j].a, xs[2 * j], acc[q]));
+    }
+#pragma unroll
+  for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+    for (int j = 0; j < JA; ++j)
+      if (j < JA - 1 || in) *reinterpret_cast<Pair<T>*>(row0 + q * ldr + c0 + 2 * j * NT) = e[q][j];
 }
 
 // kUpperInPlace: the variant that reads the upper triangle of p.afull (== p.aout) in place instead of a full
 // symmetric copy, and therefore waits at one grid barrier after loading, before any CTA writes the matrix.
-// kSmemRows: rows resident in shared memory (known at compile time, so row accesses are shared-memory instructions).
-template <typename T, int NT, int CPT, bool kUpperInPlace = false, bool kSmemRows = true>
+// kSmemRows: rows from RR on are resident in shared memory (known at compile time, so row accesses are shared-memory
+// instructions).  CPT columns per thread in pairs; NT CPT >= n.
+template <typename T, int NT, int CPT, int RR, bool kUpperInPlace = false, bool kSmemRows = true>
 __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p) {
-  constexpr int NW = NT / 32;
+  constexpr int NW = NT / 32, CP = CPT / 2;
+  static_assert(RR == 0 || RR == 4 || RR == 8, "register rows: whole, half or none of a reduce-scatter");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int G = gridDim.x, cta = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int n = p.n, R = p.rows_per_cta;
-  const size_t ldr = (size_t)p.ldr;
+  const int n = p.n, R = p.rows_per_cta, H = p.ring_h;
+  const size_t ldr = (size_t)p.ldr, slot_ld = sytrd_ring_elems(n, 1) / 3;
   if (ld_volatile_i32(&p.st->code) != 0) return;  // an earlier stage failed: every CTA skips the reduction
+  constexpr int BL = sytrd_row_block<T>();
+  auto row_of = [&](int q) { return BL * ((q / BL) * G + cta) + (q % BL); };
 
-  T* red = reinterpret_cast<T*>(smem_raw);  // [R][NW] per-warp partial row sums
-  T* vrow = red + (size_t)R * NW;           // [R] previous v at own rows
-  T* yrow = vrow + R;                       // [R] previous y at own rows (with vrow: the previous w at own rows)
-  T* colk = yrow + R;                       // [R] A(r, k-1) captured by the pass
-  T* bred = colk + R;                       // [3][NW] block-reduction scratch (rotated)
-  T* scal = bred + 3 * NW;                  // [8] broadcast scalars
-  T* rows;
+  // Shared memory (sytrd_smem_bytes): x, (v, y) at own rows, per-warp partial row sums, captured A(r, k-1), block
+  // sums, broadcast scalars, rows.
+  T* xsm = reinterpret_cast<T*>(smem_raw);                   // [NT * CPT] x of this column
+  Pair<T>* vy = reinterpret_cast<Pair<T>*>(xsm + NT * CPT);  // [R + 8] previous (v, y), zero beyond R
+  T* red = reinterpret_cast<T*>(vy + R + 8);                 // [NW][R + 8]
+  T* colk = red + (size_t)(R + 8) * NW;                      // [8]
+  T* bred = colk + 8;                                        // [2][NW]
+  T* scal = bred + 2 * NW;                                   // [4]
+  T* rows = nullptr;
   if constexpr (kSmemRows) {
-    size_t off = (size_t)(R * NW + 3 * R + 3 * NW + 8) * sizeof(T);
-    off = (off + 15) & ~size_t(15);
-    rows = reinterpret_cast<T*>(smem_raw + off);
+    const size_t off = (size_t)(reinterpret_cast<unsigned char*>(scal + 4) - smem_raw);
+    rows = reinterpret_cast<T*>(smem_raw + ((off + 15) & ~size_t(15)));
   } else {
     rows = p.grows + (size_t)cta * R * ldr;
   }
 
   // Load own rows (row r of the symmetric matrix is its column r: contiguous).
-  for (int q = 0; q < R; ++q) {
-    const int r = cta + q * G;
-    if (r >= n) break;
-    const T* src = p.afull + (size_t)r * p.ldf;
-    T* dst = rows + q * ldr;
-    if constexpr (kUpperInPlace) {
-      for (int c = tid; c < n; c += NT) dst[c] = c <= r ? src[c] : p.afull[r + (size_t)c * p.ldf];
-    } else {
-      for (int c = tid; c < n; c += NT) dst[c] = src[c];
+  T ra[RR > 0 ? RR : 1][CPT];
+  auto load = [&](int r, int c) -> T {
+    if constexpr (kUpperInPlace)
+      return c <= r ? p.afull[c + (size_t)r * p.ldf] : p.afull[r + (size_t)c * p.ldf];
+    else
+      return p.afull[c + (size_t)r * p.ldf];
+  };
+#pragma unroll
+  for (int q = 0; q < RR; ++q) {
+    const int r = row_of(q);
+#pragma unroll
+    for (int i = 0; i < CPT; ++i) {
+      const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+      ra[q][i] = (r < n && c < n) ? load(r, c) : T(0);
     }
   }
-
-  T x[CPT], vn[CPT], vk[CPT], wk[CPT];
-  int own_q[CPT];  // local row index when this thread's column c is also a row of this CTA, else -1
-#pragma unroll
-  for (int j = 0; j < CPT; ++j) {
-    const int c = tid + j * NT;
-    own_q[j] = (c % G == cta) ? c / G : -1;
-    x[j] = (n >= 1 && c < n - 1) ? p.afull[c + (size_t)(n - 1) * p.ldf] : T(0);
-    vk[j] = wk[j] = vn[j] = T(0);
+  for (int q = RR; q < R; ++q) {
+    const int r = row_of(q);
+    if (r >= n) break;
+    T* dst = rows + (size_t)(q - RR) * ldr;
+    for (int c = tid; c < (int)ldr; c += NT) dst[c] = c < n ? load(r, c) : T(0);
   }
+
+  T xs[CPT], vk[CPT], wk[CPT];
+#pragma unroll
+  for (int i = 0; i < CPT; ++i) {
+    const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+    const T x = (n >= 1 && c < n - 1) ? load(n - 1, c) : T(0);
+    xsm[c] = x;
+    if (c == n - 2) scal[0] = x;
+    xs[i] = c < n - 2 ? x : T(0);
+    vk[i] = wk[i] = T(0);
+  }
+  for (int q = tid; q < R + 8; q += NT) vy[q] = Pair<T>{T(0), T(0)};
   if (cta == 0 && tid == 0 && n >= 1) {
-    T dn = p.afull[(size_t)(n - 1) + (size_t)(n - 1) * p.ldf];
+    T dn = load(n - 1, n - 1);
     p.d[n - 1] = dn;
     p.aout[(size_t)(n - 1) + (size_t)(n - 1) * p.lda] = dn;
   }
   __syncthreads();
-
-  unsigned epoch = 0;
-  const unsigned members = (unsigned)(G + p.extra_members);
   if constexpr (kUpperInPlace) {
-    if (!group_barrier(p.counter, members, epoch, p.st, p.limit_ns)) return;
+    unsigned epoch = 0;
+    if (!group_barrier(p.counter, (unsigned)G, epoch, p.st, p.limit_ns)) return;
   }
-  // tau and tau^2/2 (y.v) of the previous step: with the previous step's y at own rows (yrow) and v (vrow) they give
-  // its w at own rows, w = tau y - half v, exactly as the owner of each column forms w.
-  T tau_prev = T(0), half_prev = T(0);
-  const int k_end = p.k_stop > 0 ? p.k_stop + 1 : 1;  // last step this kernel runs
-  for (int k = n - 1; k >= k_end; --k) {
-    const int t = n - 1 - k;                   // step index
-    T* xch = p.xch + (size_t)(t & 1) * 2 * n;  // (y, column) pairs of this step
-    const bool has_prev = (k < n - 1);
-    // ---- 1. ||x||^2 of x = A(0:k-2, k) as per-warp partials, summed after the pass's __syncthreads; alpha = x(k-1).
-    //      The pass multiplies by x itself: y = A v = scale A(:, 0:k-2) x + A(:, k-1) with v = (scale x, 1), so the
-    //      Householder scalars are needed only after the pass, off the path in front of it.
-    const int tk = (k - 1) % NT, jk = (k - 1) / NT;
-    T part = T(0);
-    T xs[CPT];
-#pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      const int c = tid + j * NT;
-      xs[j] = c < k - 1 ? x[j] : T(0);
-      part = fma(xs[j], xs[j], part);
-      if (tid == tk && j == jk) scal[0] = x[j];
-    }
-    part = warp_sum(part);
-    if (lane == 0) bred[warp] = part;
 
-    // ---- 2. fused pass: previous rank-2 update + A x over own rows r < k.
-    for (int q0 = 0; q0 < R; q0 += kRowChunk) {
-      if (cta + q0 * G >= k) break;
-      T acc[kRowChunk];
+  // tau and tau^2/2 (y.v) of the previous step: with the previous step's (v, y) at own rows they give its w at own
+  // rows, w = tau y - half v, exactly as the owner of each column forms w.
+  T tau_prev = T(0), half_prev = T(0);
+  bool dead = false;  // a wait ran out or another CTA failed: this thread polls no more (the status word is set)
+  int phase = 0, third = 2;  // step index mod H; third emptied at phase 1
+  bool first_block = true;
+  const int k_end = p.k_stop > 0 ? p.k_stop + 1 : 1;  // last step this kernel runs
+  int nq = 0;                                          // own rows r < k (ascending, so they retire from the end)
+  while (nq < R && row_of(nq) < n - 1) ++nq;
+  int last_row = nq > 0 ? row_of(nq - 1) : -1;
+  int ja = (n - 1 + 2 * NT - 1) / (2 * NT);  // column pairs per thread that reach below k
+  T* xch = p.xch;                            // ((A x)_r, A(r, k-1)) pairs of this step
+  T* const ring_end = p.xch + (size_t)3 * H * slot_ld;
+  for (int k = n - 1; k >= k_end; --k) {
+    if (last_row >= k) {
+      --nq;
+      last_row = nq > 0 ? row_of(nq - 1) : -1;
+    }
+    if (2 * NT * (ja - 1) >= k) --ja;
+
+    // One column, over the first JA column pairs of every thread (the others lie beyond k).
+    auto step = [&](auto JA) {
+      constexpr int J = decltype(JA)::value, E = 2 * J;
+      // ||x||^2 of x = A(0:k-2, k): per-warp partials, summed after the pass's __syncthreads.
+      T part;
+      {
+        T s0 = T(0), s1 = T(0);
 #pragma unroll
-      for (int qq = 0; qq < kRowChunk; ++qq) {
-        acc[qq] = T(0);
-        const int q = q0 + qq;
-        const int r = cta + q * G;
-        if (q < R && r < k) {
-          T* row = rows + q * ldr;
-          const T vr = vrow[q], wr = fma(tau_prev, yrow[q], -(half_prev * vr));  // bit for bit the owner's w
+        for (int i = 0; i < E; i += 2) {
+          s0 = fma(xs[i], xs[i], s0);
+          s1 = fma(xs[i + 1], xs[i + 1], s1);
+        }
+        part = warp_sum_mma(s0 + s1);
+      }
+      // ---- 1 + 2. fused pass: previous rank-2 update + A x over own rows r < k.  Register rows beyond nq and columns
+      //      from k on need no test: v, w and x are zero there, and no one reads the sums.
+      if constexpr (RR > 0) {
+        T acc[kRowChunk];
 #pragma unroll
-          for (int j = 0; j < CPT; ++j) {
-            const int c = tid + j * NT;
-            if (c < k) {
-              T a = row[c];
-              if (has_prev) {
-                a = fma(-vr, wk[j], a);
-                a = fma(-wr, vk[j], a);
-                row[c] = a;
-              }
-              acc[qq] = fma(a, xs[j], acc[qq]);
+        for (int q = 0; q < kRowChunk; ++q) acc[q] = T(0);
+        if constexpr (RR == 8) {
+          if (nq > 4) pass_registers<8, J, CPT, T>(ra, vy, tau_prev, half_prev, wk, vk, xs, acc);
+          else if (nq > 2) pass_registers<4, J, CPT, T>(ra, vy, tau_prev, half_prev, wk, vk, xs, acc);
+          else pass_registers<2, J, CPT, T>(ra, vy, tau_prev, half_prev, wk, vk, xs, acc);
+          warp_row_sums<8>(acc, red + warp * (R + 8));
+        } else {
+          if (nq > 2) pass_registers<4, J, CPT, T>(ra, vy, tau_prev, half_prev, wk, vk, xs, acc);
+          else pass_registers<2, J, CPT, T>(ra, vy, tau_prev, half_prev, wk, vk, xs, acc);
+          warp_row_sums<4>(acc, red + warp * (R + 8));
+        }
+      }
+      for (int q0 = RR; q0 < nq; q0 += kRowChunk) {
+        T acc[kRowChunk];
+#pragma unroll
+        for (int q = 0; q < kRowChunk; ++q) acc[q] = T(0);
+        const int rem = nq - q0;
+        T* row = rows + (size_t)(q0 - RR) * ldr;
+        const Pair<T>* o = vy + q0;
+        // Rows in pairs, so at most one row beyond nq (its storage exists: R is even); sums beyond nq are not read.
+        pass_memory<2, J, NT, T>(row, ldr, k, o, tau_prev, half_prev, wk, vk, xs, acc);
+        if (rem > 2) pass_memory<2, J, NT, T>(row + 2 * ldr, ldr, k, o + 2, tau_prev, half_prev, wk, vk, xs, acc + 2);
+        if (rem > 4) {
+          pass_memory<2, J, NT, T>(row + 4 * ldr, ldr, k, o + 4, tau_prev, half_prev, wk, vk, xs, acc + 4);
+          if (rem > 6) pass_memory<2, J, NT, T>(row + 6 * ldr, ldr, k, o + 6, tau_prev, half_prev, wk, vk, xs, acc + 6);
+          warp_row_sums<8>(acc, red + warp * (R + 8) + q0);
+        } else {
+          warp_row_sums<4>(acc, red + warp * (R + 8) + q0);
+        }
+      }
+      // A(r, k-1) of the register rows, from the thread that holds column k-1 (the others are read from the row).
+      if constexpr (RR > 0) {
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          if (tid + j * NT == (k - 1) >> 1) {
+#pragma unroll
+            for (int q = 0; q < RR; ++q) colk[q] = ((k - 1) & 1) ? ra[q][2 * j + 1] : ra[q][2 * j];
+          }
+        }
+      }
+      if (lane == 0) bred[warp] = part;
+      __syncthreads();  // publishes red, colk, the rows, the ||x||^2 partials and alpha
+      // ---- 3. publish ((A x)_r, A(r,k-1)) for own rows, one thread per row; neighbouring rows fill a 32-byte sector in
+      //      one store.  The consumer forms y_r = scale (A x)_r + A(r, k-1) with the same fma as the owner.
+      T ax_own = T(0), col_own = T(0);
+      for (int q = tid; q < nq; q += NT) {
+        const T ax = tree_sum<NW>(red + q, R + 8);
+        const T ck = q < RR ? colk[q] : rows[(size_t)(q - RR) * ldr + (k - 1)];
+        st_pair(xch + 2 * (size_t)row_of(q), published(ax), published(ck));
+        if (q == tid) { ax_own = ax; col_own = ck; }
+        else red[q] = ax;  // more rows than threads
+      }
+      // ---- 4. Householder vector (identical in every CTA: same data, same order).
+      const T xn2 = tree_sum<NW>(bred, 1);
+      const T alpha = scal[0];
+      T beta, tau, scale;
+      if (xn2 == T(0)) {
+        beta = alpha; tau = T(0); scale = T(0);
+      } else {
+        // beta = -sign(alpha) ||(alpha, x)||, tau = (beta - alpha)/beta = 1 + |alpha|/||.||: one reciprocal square
+        // root and one division.
+        const T s2 = alpha * alpha + xn2;
+        const T rn = rsqrt(s2);
+        const T nrm = s2 * rn;
+        beta = alpha >= T(0) ? -nrm : nrm;
+        tau = T(1) + fabs(alpha) * rn;
+        scale = T(1) / (alpha - beta);
+      }
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+        vk[i] = c == k - 1 ? T(1) : xs[i] * scale;  // zero from k on
+      }
+      // ---- 5. read every row's pair for this thread's columns, polling the pairs themselves.
+      T y[E], col[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+        y[i] = col[i] = T(0);
+        if (c < k) ld_pair(xch + 2 * c, y[i], col[i]);
+      }
+      // In the shadow of the loads: own rows' (v, y) and output entries, the scalars, the ring's upkeep.
+      for (int q = tid; q < nq; q += NT) {
+        const int r = row_of(q);
+        if (q != tid) {
+          ax_own = red[q];
+          col_own = rows[(size_t)(q - RR) * ldr + (k - 1)];
+        }
+        const T v = r < k - 1 ? xsm[r] * scale : T(1);
+        vy[q] = Pair<T>{v, fma(scale, ax_own, col_own)};
+        p.aout[r + (size_t)k * p.lda] = r < k - 1 ? v : beta;
+      }
+      if (cta == 0 && tid == NT - 1) { p.e[k - 1] = beta; p.tau[k - 1] = tau; }
+      if (phase == 1) {  // empty the third that every CTA has finished reading (see above)
+        if (!first_block) {
+          T* base = p.xch + (size_t)third * H * slot_ld;
+          for (int q = tid; q < R; q += NT)
+            if (row_of(q) < n)
+              for (int s = 0; s < H; ++s)
+                st_pair(base + (size_t)s * slot_ld + 2 * row_of(q), empty_value<T>(), empty_value<T>());
+        }
+        __threadfence();
+      }
+      {
+        uint64_t t0 = 0;
+        unsigned spins = 0;
+        while (!dead) {
+          bool waiting = false;
+#pragma unroll
+          for (int i = 0; i < E; ++i) waiting = waiting || is_empty(y[i]) || is_empty(col[i]);
+          if (p.extra_members && tid == 0) {  // failure-detection hook: a pair that is never published
+            T ea, eb;
+            ld_pair(xch + 2 * (size_t)n, ea, eb);
+            waiting = waiting || is_empty(ea);
+          }
+          if (!waiting) break;
+#pragma unroll
+          for (int i = 0; i < E; ++i) {
+            const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+            if (is_empty(y[i]) || is_empty(col[i])) ld_pair(xch + 2 * c, y[i], col[i]);
+          }
+          if ((++spins & 63u) == 0) {
+            if (ld_volatile_i32(&p.st->code) != 0) dead = true;
+            const uint64_t now = global_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > p.limit_ns) {
+              set_status(p.st, kStatusBarrierTimeout, 0, n - k);
+              dead = true;
             }
           }
         }
       }
-      const T rs = warp_reduce_scatter8(acc);
-      const int qrow = q0 + ((lane >> 2) & 7);
-      if ((lane & 3) == 0 && qrow < R) red[qrow * NW + warp] = rs;
-    }
-    // A(r, k-1) after the update, for the next column and for y: the warp of the thread that owns column k-1 (and just
-    // wrote it) reads it back, one row per lane, so the element loop above carries no per-element test for it.
-    if (warp == (tk >> 5)) {
       __syncwarp();
-      for (int q = lane; q < R; q += 32) {
-        if (cta + q * G >= k) break;
-        colk[q] = rows[q * ldr + (k - 1)];
-      }
-    }
-    __syncthreads();  // publishes red, colk, the ||x||^2 partials and alpha
-    // ---- 3. publish ((A x)_r, A(r,k-1)) for own rows; (A x)_r is kept in yrow until the scale is known.  The
-    //      consumer forms y_r = scale (A x)_r + A(r, k-1) with the same fma as the owner, so the Householder scalars
-    //      below are computed while the grid barrier is in flight instead of in front of it.
-    for (int q = tid; q < R; q += NT) {
-      const int r = cta + q * G;
-      if (r < k) {
-        T ax = T(0);
+      // y(k-1) and A(k-1,k-1) for w(k-1) and d(k-1), published through the same __syncthreads as y.v.
+      {
+        T s0 = T(0), s1 = T(0);
 #pragma unroll
-        for (int w = 0; w < NW; ++w) ax += red[q * NW + w];
-        yrow[q] = ax;
-        st_pair(xch + 2 * (size_t)r, ax, colk[q]);
+        for (int i = 0; i < E; ++i) {
+          const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+          y[i] = fma(scale, y[i], col[i]);
+          if (c == k - 1) { scal[1] = y[i]; scal[2] = col[i]; }
+          if (i & 1) s1 = fma(y[i], vk[i], s1);
+          else s0 = fma(y[i], vk[i], s0);
+        }
+        const T pyv = warp_sum_mma(s0 + s1);
+        if (lane == 0) bred[NW + warp] = pyv;
       }
-    }
-    group_arrive(p.counter, epoch);
-    // ---- 4. Householder vector (identical in every CTA: same data, same order), y at own rows, v.
-    T xn2 = T(0);
+      __syncthreads();
+      const T yv = tree_sum<NW>(bred + NW, 1);
+      const T half = T(0.5) * tau * tau * yv;
+      const T wkm1 = tau * scal[1] - half;  // v(k-1) = 1
+      if (cta == 0 && tid == NT - 1) {
+        const T dk = scal[2] - T(2) * wkm1;  // A(k-1,k-1) after this step's update
+        p.d[k - 1] = dk;
+        p.aout[(size_t)(k - 1) + (size_t)(k - 1) * p.lda] = dk;
+      }
 #pragma unroll
-    for (int w = 0; w < NW; ++w) xn2 += bred[w];
-    const T alpha = scal[0];
-    T beta, tau, scale;
-    if (xn2 == T(0)) {
-      beta = alpha; tau = T(0); scale = T(0);
+      for (int j = 0; j < J; ++j) {
+        const int c0 = 2 * (tid + j * NT);
+        Pair<T> xp;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = 2 * j + h, c = c0 + h;
+          const T w = fma(tau, y[i], -(half * vk[i]));
+          const T x = c < k - 1 ? col[i] - vk[i] * wkm1 - w : T(0);
+          if (c == k - 2) scal[0] = x;
+          xs[i] = c < k - 2 ? x : T(0);
+          wk[i] = w;
+          (h ? xp.b : xp.a) = x;
+        }
+        *reinterpret_cast<Pair<T>*>(xsm + c0) = xp;
+      }
+      tau_prev = tau;
+      half_prev = half;
+    };
+    if constexpr (CP == 1) {
+      step(std::integral_constant<int, 1>{});
+    } else if constexpr (CP == 2) {
+      if (ja == 2) step(std::integral_constant<int, 2>{});
+      else step(std::integral_constant<int, 1>{});
+    } else if constexpr (CP == 4) {
+      if (ja == 4) step(std::integral_constant<int, 4>{});
+      else if (ja == 3) step(std::integral_constant<int, 3>{});
+      else if (ja == 2) step(std::integral_constant<int, 2>{});
+      else step(std::integral_constant<int, 1>{});
     } else {
-      // beta = -sign(alpha) ||(alpha, x)||, tau = (beta - alpha)/beta = 1 + |alpha|/||.||: one reciprocal square
-      // root and one division.
-      const T s2 = alpha * alpha + xn2;
-      const T rn = rsqrt(s2);
-      const T nrm = s2 * rn;
-      beta = alpha >= T(0) ? -nrm : nrm;
-      tau = T(1) + fabs(alpha) * rn;
-      scale = T(1) / (alpha - beta);
+      if (ja > 4) step(std::integral_constant<int, CP>{});
+      else step(std::integral_constant<int, 4>{});
     }
-    for (int q = tid; q < R; q += NT) {
-      if (cta + q * G < k) yrow[q] = fma(scale, yrow[q], colk[q]);  // y_r for the next step's w at own rows
+    xch += slot_ld;
+    if (xch == ring_end) xch = p.xch;
+    if (++phase == H) {
+      phase = 0;
+      first_block = false;
+      third = third == 2 ? 0 : third + 1;
     }
-#pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      const int c = tid + j * NT;
-      vn[j] = c < k - 1 ? x[j] * scale : (c == k - 1 ? T(1) : T(0));
-      if (c < k && own_q[j] >= 0) vrow[own_q[j]] = vn[j];
-    }
-    if (cta == 0 && tid == 0) { p.e[k - 1] = beta; p.tau[k - 1] = tau; }
-    if (cta == k % G) {
-      T* col = p.aout + (size_t)k * p.lda;
-#pragma unroll
-      for (int j = 0; j < CPT; ++j) {
-        const int c = tid + j * NT;
-        if (c < k - 1) col[c] = vn[j];
-        else if (c == k - 1) col[c] = beta;
-      }
-    }
-    if (!group_wait(p.counter, members, epoch, p.st, p.limit_ns)) return;
-    T yj[CPT], colj[CPT];
-#pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      yj[j] = colj[j] = T(0);
-      if (tid + j * NT < k) {
-        T ax;
-        ld_pair(xch + 2 * (size_t)(tid + j * NT), ax, colj[j]);
-        yj[j] = fma(scale, ax, colj[j]);
-      }
-    }
-    // y(k-1) and A(k-1,k-1) for w(k-1) and d(k-1), published through the same __syncthreads as y.v.
-    T pyv = T(0);
-#pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      pyv += yj[j] * vn[j];
-      if (tid == tk && j == jk) { scal[1] = yj[j]; scal[2] = colj[j]; }
-    }
-    const T yv = block_sum_nw<NW>(pyv, bred + NW);
-    const T half = T(0.5) * tau * tau * yv;
-    const T wkm1 = tau * scal[1] - half;  // v(k-1) = 1
-    if (cta == 0 && tid == 0) {
-      const T dk = scal[2] - T(2) * wkm1;  // A(k-1,k-1) after this step's update
-      p.d[k - 1] = dk;
-      p.aout[(size_t)(k - 1) + (size_t)(k - 1) * p.lda] = dk;
-    }
-#pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      const int c = tid + j * NT;
-      const T w = fma(tau, yj[j], -(half * vn[j]));
-      x[j] = c < k - 1 ? colj[j] - vn[j] * wkm1 - w : T(0);
-      vk[j] = vn[j];
-      wk[j] = w;
-    }
-    tau_prev = tau;
-    half_prev = half;
   }
   // Hand-over: the pending update of step k_stop + 1 applied to the trailing block, whose full symmetric rows go to
-  // `hand` (row r of the block is its column r).  vrow, yrow and the scalars are this CTA's own; vk and wk were
-  // formed after the last barrier, so every row of the block is complete.
+  // `hand` (row r of the block is its column r).  vy and the scalars are this CTA's own; vk and wk were formed after
+  // the last exchange, so every row of the block is complete.
   if (p.k_stop > 0 && k_end <= n - 1) {
     const int m = p.k_stop + 1;
-    for (int q = 0; q < R; ++q) {
-      const int r = cta + q * G;
-      if (r >= m) break;
-      const T* row = rows + q * ldr;
-      const T vr = vrow[q], wr = fma(tau_prev, yrow[q], -(half_prev * vr));
+    auto hand_row = [&](int q, auto get) {
+      const int r = row_of(q);
+      const Pair<T> o = vy[q];
+      const T vr = o.a, wr = fma(tau_prev, o.b, -(half_prev * vr));
       T* dst = p.hand + (size_t)r * p.ldh;
 #pragma unroll
-      for (int j = 0; j < CPT; ++j) {
-        const int c = tid + j * NT;
-        if (c < m) dst[c] = fma(-wr, vk[j], fma(-vr, wk[j], row[c]));
+      for (int i = 0; i < CPT; ++i) {
+        const int c = 2 * (tid + (i >> 1) * NT) + (i & 1);
+        if (c < m) dst[c] = fma(-wr, vk[i], fma(-vr, wk[i], get(i, c)));
       }
-    }
+    };
+#pragma unroll
+    for (int q = 0; q < RR; ++q)
+      if (row_of(q) < m) hand_row(q, [&](int i, int) { return ra[q][i]; });
+    for (int q = RR; q < R && row_of(q) < m; ++q)
+      hand_row(q, [&](int, int c) { return rows[(size_t)(q - RR) * ldr + c]; });
   }
 }
 
@@ -430,9 +674,10 @@ __global__ void __launch_bounds__(NT, 1) sytrd_tail_kernel(SytrdParams<T> p, int
   }
 }
 
-template <typename T, int NT, int CPT>
+template <typename T, int NT, int CPT, int RR>
 cudaError_t launch_one(const SytrdParams<T>& p, int G, size_t smem, cudaStream_t s) {
-  auto kern = p.use_smem ? sytrd_resident_kernel<T, NT, CPT, false, true> : sytrd_resident_kernel<T, NT, CPT, false, false>;
+  auto kern = p.use_smem ? sytrd_resident_kernel<T, NT, CPT, RR, false, true>
+                         : sytrd_resident_kernel<T, NT, CPT, RR, false, false>;
   cudaError_t err = allow_max_dynamic_smem(kern);
   if (err != cudaSuccess) return err;
   void* args[] = {(void*)&p};
@@ -441,40 +686,49 @@ cudaError_t launch_one(const SytrdParams<T>& p, int G, size_t smem, cudaStream_t
   return err;
 }
 
-template <int CPT>
+template <int NT, int CPT, int RR>
 cudaError_t launch_upper_inplace(const SytrdParams<double>& p, int G, size_t smem, cudaStream_t s) {
-  auto kern = sytrd_resident_kernel<double, 512, CPT, true>;
+  auto kern = sytrd_resident_kernel<double, NT, CPT, RR, true>;
   cudaError_t err = allow_max_dynamic_smem(kern);
   if (err != cudaSuccess) return err;
   void* args[] = {(void*)&p};
-  err = cudaLaunchCooperativeKernel((void*)kern, dim3(G), dim3(512), args, smem, s);
+  err = cudaLaunchCooperativeKernel((void*)kern, dim3(G), dim3(NT), args, smem, s);
   note_launches();
   return err;
 }
 
+// Every slot of the ring starts empty (all ones), as far as the launch uses it.
+template <typename T>
+cudaError_t empty_ring(const SytrdParams<T>& p, cudaStream_t s) {
+  return cudaMemsetAsync(p.xch, 0xff, sytrd_ring_elems(p.n, p.ring_h) * sizeof(T), s);
+}
+
 }  // namespace
 
-// The in-place variant (upper triangle read where it lies; rows in shared memory; FP64; n <= 2048).
+// The in-place variant (upper triangle read where it lies; FP64; n <= 2048).
 cudaError_t sytrd_launch_upper_inplace(const SytrdParams<double>& p, const SytrdPlan& pl, cudaStream_t s) {
   if (p.n <= 0) return cudaSuccess;
-  if (!pl.rows_in_smem || pl.threads != 512) return cudaErrorInvalidValue;
-  switch (pl.cpt) {
-    case 2: return launch_upper_inplace<2>(p, pl.grid, pl.smem, s);
-    case 4: return launch_upper_inplace<4>(p, pl.grid, pl.smem, s);
+  if (!pl.rows_in_smem) return cudaErrorInvalidValue;
+  cudaError_t err = empty_ring(p, s);
+  if (err != cudaSuccess) return err;
+  switch (pl.threads * 1000 + pl.cpt * 10 + pl.reg_rows) {
+    case 128024: return launch_upper_inplace<128, 2, 4>(p, pl.grid, pl.smem, s);
+    case 128044: return launch_upper_inplace<128, 4, 4>(p, pl.grid, pl.smem, s);
+    case 256044: return launch_upper_inplace<256, 4, 4>(p, pl.grid, pl.smem, s);
+    case 256048: return launch_upper_inplace<256, 4, 8>(p, pl.grid, pl.smem, s);
+    case 256088: return launch_upper_inplace<256, 8, 8>(p, pl.grid, pl.smem, s);
   }
   return cudaErrorInvalidValue;
 }
 
 template <typename T>
-size_t sytrd_smem_bytes(int n, int G, int NT, bool rows_in_smem, int* R_out, int* ldr_out) {
-  const int R = (n + G - 1) / G;
+size_t sytrd_smem_bytes(int n, int R, int NT, int cpt, int smem_rows, int* ldr_out) {
   const int align = 16 / (int)sizeof(T);
   const int ldr = ((n + align - 1) / align) * align;
   const int NW = NT / 32;
-  size_t bytes = (size_t)(R * NW + 3 * R + 3 * NW + 8) * sizeof(T);
-  bytes = (bytes + 15) & ~size_t(15);
-  if (rows_in_smem) bytes += (size_t)R * ldr * sizeof(T);
-  if (R_out) *R_out = R;
+  const size_t elems = (size_t)NT * cpt + 2 * ((size_t)R + 8) + ((size_t)R + 8) * NW + 8 + 2 * (size_t)NW + 4;
+  size_t bytes = (elems * sizeof(T) + 15) & ~size_t(15);
+  bytes += (size_t)smem_rows * ldr * sizeof(T);
   if (ldr_out) *ldr_out = ldr;
   return bytes;
 }
@@ -482,19 +736,24 @@ size_t sytrd_smem_bytes(int n, int G, int NT, bool rows_in_smem, int* R_out, int
 template <typename T>
 SytrdPlan sytrd_plan(int n, int num_sms, size_t max_smem, int grid_override) {
   SytrdPlan pl{};
-  int G = grid_override > 0 ? grid_override : num_sms;
   // Small problems: fewer CTAs, at least ~4 rows each.
-  if (grid_override <= 0) G = max(1, min(G, (n + 3) / 4));
+  const int G = grid_override > 0 ? grid_override : max(1, min(num_sms, (n + 3) / 4));
   pl.grid = G;
-  pl.threads = 512;
-  pl.cpt = (n + pl.threads - 1) / pl.threads;
-  if (pl.cpt <= 2) pl.cpt = 2;
-  else if (pl.cpt <= 4) pl.cpt = 4;
-  else if (pl.cpt <= 8) pl.cpt = 8;
-  else { pl.threads = 1024; pl.cpt = (n + 1023) / 1024 <= 8 ? 8 : 16; }
-  size_t with_rows = sytrd_smem_bytes<T>(n, G, pl.threads, true, &pl.rows_per_cta, &pl.ldr);
+  // Few warps keep the block syncs and cross-warp sums short; at least four, one per scheduler.
+  if (n <= 256) { pl.threads = 128; pl.cpt = 2; }
+  else if (n <= 512) { pl.threads = 128; pl.cpt = 4; }
+  else if (n <= 1024) { pl.threads = 256; pl.cpt = 4; }
+  else if (n <= 2048) { pl.threads = 256; pl.cpt = 8; }
+  else if (n <= 4096) { pl.threads = 512; pl.cpt = 8; }
+  else { pl.threads = 1024; pl.cpt = n <= 8192 ? 8 : 16; }
+  // Registers hold the rows of a CTA that has few of them; blocks of more than 256 threads have none to spare.
+  constexpr int BL = sytrd_row_block<T>();
+  pl.rows_per_cta = BL * (((n + BL - 1) / BL + G - 1) / G);
+  const int reg_rows = pl.reg_rows = pl.threads > 256 ? 0 : pl.rows_per_cta <= 4 ? 4 : 8;
+  const int others = max(0, pl.rows_per_cta - reg_rows);
+  const size_t with_rows = sytrd_smem_bytes<T>(n, pl.rows_per_cta, pl.threads, pl.cpt, others, &pl.ldr);
   pl.rows_in_smem = with_rows <= max_smem;
-  pl.smem = pl.rows_in_smem ? with_rows : sytrd_smem_bytes<T>(n, G, pl.threads, false, nullptr, nullptr);
+  pl.smem = pl.rows_in_smem ? with_rows : sytrd_smem_bytes<T>(n, pl.rows_per_cta, pl.threads, pl.cpt, 0, nullptr);
   pl.supported = (size_t)pl.threads * pl.cpt >= (size_t)n && pl.cpt <= 16;
   return pl;
 }
@@ -502,17 +761,19 @@ SytrdPlan sytrd_plan(int n, int num_sms, size_t max_smem, int grid_override) {
 template <typename T>
 cudaError_t sytrd_launch(const SytrdParams<T>& p, const SytrdPlan& pl, cudaStream_t s) {
   if (p.n <= 0) return cudaSuccess;
-  if (pl.threads == 512) {
-    switch (pl.cpt) {
-      case 2: return launch_one<T, 512, 2>(p, pl.grid, pl.smem, s);
-      case 4: return launch_one<T, 512, 4>(p, pl.grid, pl.smem, s);
-      case 8: return launch_one<T, 512, 8>(p, pl.grid, pl.smem, s);
-    }
-  } else {
-    switch (pl.cpt) {
-      case 8: return launch_one<T, 1024, 8>(p, pl.grid, pl.smem, s);
-      case 16: return launch_one<T, 1024, 16>(p, pl.grid, pl.smem, s);
-    }
+  const cudaError_t err = empty_ring(p, s);
+  if (err != cudaSuccess) return err;
+  switch (pl.threads * 1000 + pl.cpt * 10 + pl.reg_rows) {
+    case 128024: return launch_one<T, 128, 2, 4>(p, pl.grid, pl.smem, s);
+    case 128028: return launch_one<T, 128, 2, 8>(p, pl.grid, pl.smem, s);
+    case 128044: return launch_one<T, 128, 4, 4>(p, pl.grid, pl.smem, s);
+    case 128048: return launch_one<T, 128, 4, 8>(p, pl.grid, pl.smem, s);
+    case 256044: return launch_one<T, 256, 4, 4>(p, pl.grid, pl.smem, s);
+    case 256048: return launch_one<T, 256, 4, 8>(p, pl.grid, pl.smem, s);
+    case 256088: return launch_one<T, 256, 8, 8>(p, pl.grid, pl.smem, s);
+    case 512080: return launch_one<T, 512, 8, 0>(p, pl.grid, pl.smem, s);
+    case 1024080: return launch_one<T, 1024, 8, 0>(p, pl.grid, pl.smem, s);
+    case 1024160: return launch_one<T, 1024, 16, 0>(p, pl.grid, pl.smem, s);
   }
   return cudaErrorInvalidValue;
 }
