@@ -63,11 +63,10 @@ template <typename T>
 SytrdPlan sytrd_plan(int n, int num_sms, size_t max_smem, int grid_override);
 template <typename T>
 cudaError_t sytrd_launch(const SytrdParams<T>& p, const SytrdPlan& pl, cudaStream_t s);
-// The last columns of the reduction on one CTA: the leading m x m block (m = p.n), full symmetric rows in p.afull
-// (ld p.ldf; the whole matrix, or a grid launch's hand-over), reduced in shared memory with block-level syncs only.
-// Writes d(0:m-1) (d(m-1) only when skip_dinit is 0), e, tau and the reflector columns 1..m-1 of p.aout.
-template <typename T>
-size_t sytrd_tail_smem(int m);
+// The last columns of the reduction on one CTA: the leading m x m block (m = p.n <= kSytrdTailMax), full symmetric rows
+// in p.afull (ld p.ldf; the whole matrix, or a grid launch's hand-over), reduced in registers with one block sync per
+// column.  Writes d(0:m-1) (d(m-1) only when skip_dinit is 0), e, tau and the reflector columns 1..m-1 of p.aout.
+constexpr int kSytrdTailMax = 128;
 template <typename T>
 cudaError_t sytrd_tail_launch(const SytrdParams<T>& p, int skip_dinit, cudaStream_t s);
 // Variant reading the upper triangle of p.afull == p.aout in place (FP64, rows in shared memory, n <= 2048).

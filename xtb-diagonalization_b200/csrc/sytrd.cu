@@ -572,105 +572,213 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
   }
 }
 
-// The last columns on one CTA.  The trailing block's upper triangle lives in shared memory with an odd leading
-// dimension (row- and column-strided reads spread over the banks) and is updated symmetrically; per column k:
-//   1. every warp sums ||x||^2 of x = A(0:k-2, k) itself (the same lanes and shuffle tree in every warp, so all warps
-//      hold the same value without a block sync), every thread forms beta, tau and scale as the grid kernel does, and
-//      threads c < k write v(c) and the output column;
-//   2. y = A v with four threads per row (row r read along the row for c >= r and down the column for c < r);
-//   3. every warp sums y.v itself; threads r < k form w = tau y - tau^2/2 (y.v) v;
-//   4. the rank-2 update A -= v w^T + w v^T of the upper triangle, eight threads per pair of rows (r, k-1-r).
-// Four block syncs per column and no grid barrier: where the trailing matrix is small the grid kernel's per-column
-// exchange costs more than the work.  Sums run in a fixed order, so results are deterministic.
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT, 1) sytrd_tail_kernel(SytrdParams<T> p, int skip_dinit) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int m = p.n, ld = (m & 1) ? m + 2 : m + 1;
-  T* A = reinterpret_cast<T*>(smem_raw);  // upper triangle, A[r * ld + c] for r <= c
-  T* v = A + (size_t)m * ld;
-  T* y = v + m;
-  T* w = y + m;
-  const int tid = threadIdx.x, lane = tid & 31;
+// Reduce-scatter of ROWS (16, 8 or 4) per-lane values per warp: the warp-wide sum of row i to out[i * stride].  Halves
+// are exchanged across lanes 16, 8, 4 as in warp_row_sums; one matrix instruction then sums the quads of each value
+// that is left (16 rows leave two per lane).
+template <int ROWS>
+__device__ __forceinline__ void warp_row_sums_strided(double (&acc)[ROWS], double* out, int stride) {
+  const unsigned lane = threadIdx.x & 31;
+  int rows = ROWS;
+#pragma unroll
+  for (int bit = 16; bit >= 4; bit /= 2) {
+    const bool hi = lane & bit;
+    if (rows > 1) {
+#pragma unroll
+      for (int i = 0; i < ROWS / 2; ++i) {
+        if (i < rows / 2) {
+          const double send = hi ? acc[i] : acc[i + rows / 2], keep = hi ? acc[i + rows / 2] : acc[i];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+      }
+      rows /= 2;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], bit);
+    }
+  }
+  // Quad n (lanes 4n .. 4n + 3) now holds rows n ROWS/8 + s (ROWS 4: row n / 2).
+  constexpr int S = ROWS >= 8 ? ROWS / 8 : 1;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    double even, odd;
+    quad_sums(acc[s], even, odd);
+    if (lane < 4) {
+      if constexpr (ROWS == 4) {
+        out[lane * stride] = even;
+      } else {
+        out[(2 * lane * S + s) * stride] = even;
+        out[((2 * lane + 1) * S + s) * stride] = odd;
+      }
+    }
+  }
+}
+template <int ROWS>
+__device__ __forceinline__ void warp_row_sums_strided(float (&acc)[ROWS], float* out, int stride) {
+  const unsigned lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const float r = warp_sum(acc[i]);
+    if (lane == (unsigned)i) out[i * stride] = r;
+  }
+}
+
+// The last columns on one CTA, the trailing block (order m <= M) in registers: warp w of M / 16 owns rows w, w + NW, ...
+// (16 of them), lane l the columns l, l + 32, ...  Per column k, as in the grid kernel: the pass applies the previous
+// rank-2 update and sums A x at the warp's rows; one block sync exchanges (A x)_r and A(r, k-1) through shared memory
+// (two alternating buffers); every warp then forms y, v, w and the next x itself, from the same data in the same order,
+// so no other sync is needed.  For M = 64 one more warp owns no rows: it forms the Householder scalars of the same x while
+// the others pass over their rows (a dependent chain of a sum, a reciprocal square root and a division).
+// A warp's own copy of (v, w) in shared memory gives it the values at its rows.  Bound by latency: the pass and its
+// reduce-scatter, one sync, a warp sum by matrix instruction.  It replaced a kernel that kept the block in shared memory
+// with four block syncs and two shuffled sums per column (2.0 us per column of a block of 64, now 0.7: 130 -> 45 us).
+template <typename T, int M>
+__global__ void __launch_bounds__(2 * M + (M == 64 ? 32 : 0), 1) sytrd_tail_kernel(SytrdParams<T> p, int skip_dinit) {
+  constexpr int NW = M / 16, CJ = M / 32;
+  constexpr bool kScalarWarp = M == 64;  // M = 128: the registers of a ninth warp would make the others spill
+  __shared__ Pair<T> vw[NW][M];  // each warp's (v, w)
+  __shared__ T ax_s[2][M], col_s[2][M], scal_s[2][4];
+  const int m = p.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (ld_volatile_i32(&p.st->code) != 0) return;  // an earlier stage failed
-  for (int idx = tid; idx < m * m; idx += NT) {
-    const int r = idx / m, c = idx - r * m;
-    if (r <= c) A[r * ld + c] = p.afull[(size_t)r * p.ldf + c];
+  T a[16][CJ], x[CJ], v[CJ], w[CJ];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = warp + NW * i;
+#pragma unroll
+    for (int j = 0; j < CJ; ++j) {
+      const int c = lane + 32 * j;
+      a[i][j] = (warp < NW && r < m && c < m) ? p.afull[(size_t)r * p.ldf + c] : T(0);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < CJ; ++j) {
+    const int c = lane + 32 * j;
+    x[j] = (m >= 2 && c < m - 1) ? p.afull[(size_t)(m - 1) * p.ldf + c] : T(0);
+    v[j] = w[j] = T(0);
+    if (warp < NW) vw[warp][c] = Pair<T>{T(0), T(0)};
   }
   if (!skip_dinit && tid == 0 && m >= 1) {
     const T dn = p.afull[(size_t)(m - 1) * p.ldf + (m - 1)];
     p.d[m - 1] = dn;
     p.aout[(size_t)(m - 1) + (size_t)(m - 1) * p.lda] = dn;
   }
-  __syncthreads();
-  const int sub4 = tid & 3;
-  const unsigned qmask = 0xFu << (lane & ~3);
+  __syncwarp();
   for (int k = m - 1; k >= 1; --k) {
-    // 1. Householder vector.
-    T part = T(0);
-    for (int c = lane; c < k - 1; c += 32) part = fma(A[c * ld + k], A[c * ld + k], part);
-    const T xn2 = warp_sum(part);
-    const T alpha = A[(k - 1) * ld + k];
-    T beta, tau, scale;
-    if (xn2 == T(0)) {
-      beta = alpha; tau = T(0); scale = T(0);
-    } else {
-      const T s2 = alpha * alpha + xn2;
-      const T rn = rsqrt(s2);
-      const T nrm = s2 * rn;
-      beta = alpha >= T(0) ? -nrm : nrm;
-      tau = T(1) + fabs(alpha) * rn;
-      scale = T(1) / (alpha - beta);
-    }
-    for (int c = tid; c < k; c += NT) {
-      const T vc = c < k - 1 ? A[c * ld + k] * scale : T(1);
-      v[c] = vc;
-      p.aout[(size_t)c + (size_t)k * p.lda] = c < k - 1 ? vc : beta;
-    }
-    if (tid == 0) { p.e[k - 1] = beta; p.tau[k - 1] = tau; }
-    __syncthreads();
-    // 2. y = A v.
-    for (int r = tid >> 2; r < k; r += NT / 4) {
-      T a0 = T(0), a1 = T(0);
-      int c = sub4;
-      for (; c < r; c += 4) a0 = fma(A[c * ld + r], v[c], a0);
-      for (; c < k; c += 4) a1 = fma(A[r * ld + c], v[c], a1);
-      T sum = a0 + a1;
-      sum += __shfl_xor_sync(qmask, sum, 1);
-      sum += __shfl_xor_sync(qmask, sum, 2);
-      if (sub4 == 0) y[r] = sum;
-    }
-    __syncthreads();
-    // 3. y.v and w; d(k-1) = A(k-1,k-1) - 2 w(k-1) (v(k-1) = 1).
-    T pv = T(0);
-    for (int r = lane; r < k; r += 32) pv = fma(y[r], v[r], pv);
-    const T yv = warp_sum(pv);
-    const T half = T(0.5) * tau * tau * yv;
-    for (int r = tid; r < k; r += NT) w[r] = fma(tau, y[r], -(half * v[r]));
-    if (tid == 0) {
-      const T wkm1 = tau * y[k - 1] - half;
-      const T dk = A[(k - 1) * ld + (k - 1)] - T(2) * wkm1;
-      p.d[k - 1] = dk;
-      p.aout[(size_t)(k - 1) + (size_t)(k - 1) * p.lda] = dk;
-    }
-    __syncthreads();
-    // 4. Rank-2 update of the upper triangle of A(0:k-1, 0:k-1): group g of eight threads takes rows g and k-1-g.
-    {
-      const int g = tid >> 3, sub8 = tid & 7;
-      for (int gg = g; 2 * gg < k; gg += NT / 8) {
-        for (int h = 0; h < 2; ++h) {
-          const int r = h == 0 ? gg : k - 1 - gg;
-          if (h == 1 && r == gg) break;
-          const T vr = v[r], wr = w[r];
-          for (int c = r + sub8; c < k; c += 8) {
-            T a = A[r * ld + c];
-            a = fma(-vr, w[c], a);
-            a = fma(-wr, v[c], a);
-            A[r * ld + c] = a;
+    // One column over the first J column groups and ROWS rows per warp (the others lie beyond k).
+    auto step = [&](auto Jc, auto Rc) {
+      constexpr int J = decltype(Jc)::value, ROWS = decltype(Rc)::value;
+      const int buf = k & 1, lk = (k - 1) & 31, jk = (k - 1) >> 5;
+      T xs[J];
+#pragma unroll
+      for (int j = 0; j < J; ++j) xs[j] = lane + 32 * j < k - 1 ? x[j] : T(0);
+      // ||x(0:k-2)||^2, alpha = x(k-1) and the Householder scalars.
+      T beta, tau, scale;
+      auto scalars = [&]() {
+        T part = T(0), alpha = T(0);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          part = fma(xs[j], xs[j], part);
+          if (j == jk) alpha = __shfl_sync(0xffffffffu, x[j], lk);
+        }
+        const T xn2 = warp_sum_mma(part);
+        if (xn2 == T(0)) {
+          beta = alpha; tau = T(0); scale = T(0);
+        } else {
+          const T s2 = alpha * alpha + xn2;
+          const T rn = rsqrt(s2);
+          const T nrm = s2 * rn;
+          beta = alpha >= T(0) ? -nrm : nrm;
+          tau = T(1) + fabs(alpha) * rn;
+          scale = T(1) / (alpha - beta);
+        }
+      };
+      if (warp < NW) {
+        // Previous rank-2 update and A x at own rows (v = w = x = 0 beyond the block).
+        T acc[ROWS];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+          const Pair<T> o = vw[warp][warp + NW * i];
+          acc[i] = T(0);
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            T e = fma(-o.a, w[j], a[i][j]);
+            e = fma(-o.b, v[j], e);
+            a[i][j] = e;
+            acc[i] = fma(e, xs[j], acc[i]);
           }
         }
+        // A(r, k-1) of own rows, from the lane that holds column k-1.
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          if (j == jk) {
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i)
+              if (lane == lk) col_s[buf][warp + NW * i] = a[i][j];
+          }
+        }
+        warp_row_sums_strided<ROWS>(acc, &ax_s[buf][warp], NW);
+      } else {
+        scalars();
+        if (lane == 0) {
+          scal_s[buf][0] = tau;
+          scal_s[buf][1] = scale;
+          scal_s[buf][2] = beta;
+        }
       }
+      if constexpr (!kScalarWarp) scalars();
+      __syncthreads();
+      if constexpr (kScalarWarp) {
+        tau = scal_s[buf][0];
+        scale = scal_s[buf][1];
+        beta = scal_s[buf][2];
+      }
+      T y[J], col[J], pyv = T(0), yk = T(0), ck = T(0);
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int c = lane + 32 * j;
+        const bool in = c < k;
+        col[j] = in ? col_s[buf][c] : T(0);
+        y[j] = in ? fma(scale, ax_s[buf][c], col[j]) : T(0);
+        v[j] = c == k - 1 ? T(1) : xs[j] * scale;
+        pyv = fma(y[j], v[j], pyv);
+        if (j == jk) {
+          yk = __shfl_sync(0xffffffffu, y[j], lk);
+          ck = col[j];
+        }
+      }
+      const T half = T(0.5) * tau * tau * warp_sum_mma(pyv);
+      const T wkm1 = tau * yk - half;  // v(k-1) = 1
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int c = lane + 32 * j;
+        w[j] = fma(tau, y[j], -(half * v[j]));
+        x[j] = c < k - 1 ? col[j] - v[j] * wkm1 - w[j] : T(0);
+        if (warp < NW) vw[warp][c] = Pair<T>{v[j], w[j]};
+      }
+      __syncwarp();
+      if (warp == (kScalarWarp ? NW : k % NW)) {  // the output column
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const int c = lane + 32 * j;
+          if (c < k) p.aout[(size_t)c + (size_t)k * p.lda] = c < k - 1 ? v[j] : beta;
+        }
+        if (lane == lk) {
+          const T dk = ck - T(2) * wkm1;  // A(k-1,k-1) after this step's update
+          p.e[k - 1] = beta;
+          p.tau[k - 1] = tau;
+          p.d[k - 1] = dk;
+          p.aout[(size_t)(k - 1) + (size_t)(k - 1) * p.lda] = dk;
+        }
+      }
+    };
+    using std::integral_constant;
+    if constexpr (CJ == 4) {
+      if (k > 96) step(integral_constant<int, 4>{}, integral_constant<int, 16>{});
+      else if (k > 64) step(integral_constant<int, 3>{}, integral_constant<int, 16>{});
+      else if (k > 32) step(integral_constant<int, 2>{}, integral_constant<int, 8>{});
+      else step(integral_constant<int, 1>{}, integral_constant<int, 4>{});
+    } else {
+      if (k > 32) step(integral_constant<int, 2>{}, integral_constant<int, 16>{});
+      else step(integral_constant<int, 1>{}, integral_constant<int, 8>{});
     }
-    __syncthreads();
   }
 }
 
@@ -779,24 +887,15 @@ cudaError_t sytrd_launch(const SytrdParams<T>& p, const SytrdPlan& pl, cudaStrea
 }
 
 template <typename T>
-size_t sytrd_tail_smem(int m) {
-  const int ld = (m & 1) ? m + 2 : m + 1;
-  return ((size_t)m * ld + 3 * (size_t)m) * sizeof(T);
-}
-
-template <typename T>
 cudaError_t sytrd_tail_launch(const SytrdParams<T>& p, int skip_dinit, cudaStream_t s) {
   if (p.n <= 0) return cudaSuccess;
-  auto kern = sytrd_tail_kernel<T, 512>;
-  cudaError_t err = allow_max_dynamic_smem(kern);
-  if (err != cudaSuccess) return err;
-  kern<<<1, 512, sytrd_tail_smem<T>(p.n), s>>>(p, skip_dinit);
+  if (p.n > kSytrdTailMax) return cudaErrorInvalidValue;
+  if (p.n <= 64) sytrd_tail_kernel<T, 64><<<1, 160, 0, s>>>(p, skip_dinit);
+  else sytrd_tail_kernel<T, 128><<<1, 256, 0, s>>>(p, skip_dinit);
   note_launches();
   return cudaGetLastError();
 }
 
-template size_t sytrd_tail_smem<double>(int);
-template size_t sytrd_tail_smem<float>(int);
 template cudaError_t sytrd_tail_launch<double>(const SytrdParams<double>&, int, cudaStream_t);
 template cudaError_t sytrd_tail_launch<float>(const SytrdParams<float>&, int, cudaStream_t);
 template SytrdPlan sytrd_plan<double>(int, int, size_t, int);
