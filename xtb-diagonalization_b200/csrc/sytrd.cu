@@ -39,8 +39,8 @@
 //
 // The ring has three thirds of H slots; step t uses slot t mod 3H.  In step t = bH + 1, after publishing, the owner
 // of a row puts the empty pattern back into its entries of third (b - 1) mod 3 and every thread executes a fence.
-// Every CTA has then read all of third (b - 1) mod 3 (it published step t - 1 = bH only after reading step bH - 1,
-// and this CTA has read its step bH).  The third is polled again from step (b + 2)H on; by then the reader has seen
+// Every CTA has then read all of third (b - 1) mod 3: a CTA reads step s only if it has a row in step s + 1, which it
+// publishes after reading, and this CTA has read every pair of step t - 1 = bH.  The third is polled again from step (b + 2)H on; by then the reader has seen
 // a later publish of the same owner thread (step bH + 2 or later, H >= 2) and executed its own fence of step
 // (b + 1)H + 1, so the emptying happens before the poll.  A fence costs about 1000 cycles while stores are in flight,
 // so a third has 32 slots (8: 2 % slower).
@@ -322,6 +322,8 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
   int nq = 0;                                          // own rows r < k (ascending, so they retire from the end)
   while (nq < R && row_of(nq) < n - 1) ++nq;
   int last_row = nq > 0 ? row_of(nq - 1) : -1;
+  const int first_row = row_of(0);
+  if (first_row >= n - 1 && cta > 0) return;  // no row in any step
   int ja = (n - 1 + 2 * NT - 1) / (2 * NT);  // column pairs per thread that reach below k
   T* xch = p.xch;                            // ((A x)_r, A(r, k-1)) pairs of this step
   T* const ring_end = p.xch + (size_t)3 * H * slot_ld;
@@ -454,6 +456,10 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
         }
         __threadfence();
       }
+      // A CTA without a row in the next step is done: it must not read this step's pairs, because nothing would tell
+      // the others when it has finished, and they empty the slot some steps later.  (Row 0's CTA stays to the end, and
+      // the last step's pairs are not emptied.)
+      if (first_row >= k - 1 && k > k_end) return false;
       {
         uint64_t t0 = 0;
         unsigned spins = 0;
@@ -525,21 +531,24 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
       }
       tau_prev = tau;
       half_prev = half;
+      return true;
     };
+    bool more;
     if constexpr (CP == 1) {
-      step(std::integral_constant<int, 1>{});
+      more = step(std::integral_constant<int, 1>{});
     } else if constexpr (CP == 2) {
-      if (ja == 2) step(std::integral_constant<int, 2>{});
-      else step(std::integral_constant<int, 1>{});
+      if (ja == 2) more = step(std::integral_constant<int, 2>{});
+      else more = step(std::integral_constant<int, 1>{});
     } else if constexpr (CP == 4) {
-      if (ja == 4) step(std::integral_constant<int, 4>{});
-      else if (ja == 3) step(std::integral_constant<int, 3>{});
-      else if (ja == 2) step(std::integral_constant<int, 2>{});
-      else step(std::integral_constant<int, 1>{});
+      if (ja == 4) more = step(std::integral_constant<int, 4>{});
+      else if (ja == 3) more = step(std::integral_constant<int, 3>{});
+      else if (ja == 2) more = step(std::integral_constant<int, 2>{});
+      else more = step(std::integral_constant<int, 1>{});
     } else {
-      if (ja > 4) step(std::integral_constant<int, CP>{});
-      else step(std::integral_constant<int, 4>{});
+      if (ja > 4) more = step(std::integral_constant<int, CP>{});
+      else more = step(std::integral_constant<int, 4>{});
     }
+    if (!more) return;
     xch += slot_ld;
     if (xch == ring_end) xch = p.xch;
     if (++phase == H) {
