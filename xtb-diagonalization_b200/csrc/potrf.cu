@@ -16,6 +16,7 @@
 // A pivot that is not > 0 (or NaN) records kStatusNotSPD with the global column (1-based), LAPACK's info, and every
 // CTA leaves at the next barrier.  Every barrier wait is time-limited.
 #include <algorithm>
+#include <type_traits>
 
 #include "gemm_tile.cuh"
 #include "kernels.h"
@@ -39,244 +40,223 @@ struct PotrfParams {
   uint64_t limit_ns;
 };
 
-constexpr size_t kLeafElems = (size_t)2 * NB * (NB + 1) + NB + 8;  // U, X, 1 / U(k, k), a flag
+constexpr int kLeafLd = NB + 4;  // 4 (mod 16): fragment loads of a half warp hit 16 distinct 8-byte banks
+constexpr size_t kLeafElems = (size_t)NB * kLeafLd + NB + 4;  // rows, U(k, k), row counter and flag
 constexpr size_t kSmemBytes = (tile::smem_elems<double>() + kLeafElems) * sizeof(double);
+static_assert((size_t)NB * kLeafLd <= tile::smem_elems<double>(), "the panel fits the tile pipeline's region");
+
+// 1 / sqrt(d) for d > 0 without a branch, so that the pivot chain interleaves with the row updates: the hardware's
+// approximation y and one third-order step, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - d y^2 (the series of (1 - e)^(-1/2); the
+// approximation's error cubed is far below the last bit).  The approximation flushes subnormal arguments, so small d
+// are scaled by 2^200 first.
+__device__ __forceinline__ double pivot_rsqrt(double d) {
+  const bool small = d < 1e-250;
+  const double ds = small ? d * 0x1p200 : d;
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(ds));
+  const double e = fma(-ds * y, y, 1.0);
+  const double r = fma(y * e, fma(0.375, e, 0.5), y);
+  return small ? r * 0x1p100 : r;
+}
+
+// Elimination steps k = 16 b .. 16 b + 15 of the leaf (see leaf_factor_invert) on the 16 rows of one warp: its owner,
+// warp b, leaves the final rows in `rows` and counts them in *done, two at a time; the warps below follow.  Both are
+// rolled loops of about a hundred instructions: unrolled over the 64 steps the code, run once per leaf, was bound by
+// instruction fetch (twice the time).
+// The pivot state of the owner warp, the same in every lane: d = M(k, k), r = 1 / sqrt(d), and the two values the next
+// pivot follows from, a = M(k, k+1) and b = M(k+1, k+1): d' = b - (a r)^2 needs no shuffle once r is known.
+struct LeafPivot {
+  double d, r, a, b;
+  int bad;  // first pivot of this block that is not > 0
+};
+
+// kSecond: column k lies in the lanes' second column.  Q0: first of the 16 steps; ROWS: rows below the pivot that may
+// still be unfinished (15 in the first eight steps, 7 in the last eight).
+template <bool kSecond, int Q0, int ROWS>
+__device__ __forceinline__ void leaf_own_steps(double (&m)[16][2], LeafPivot& v, int blk, double* rows, double* diag,
+                                               volatile int* done, int lane) {
+  const int l0 = (16 * blk) & 31;
+#pragma unroll 1
+  for (int q = Q0; q < Q0 + 8; ++q) {
+    // The pivot row is m[0]: every update writes its row one place up.
+    const int k = 16 * blk + q;
+    const bool at = lane == l0 + q;
+    const double r = v.r, u1 = v.a * r;
+    v.bad = (!(v.d > 0.0) && v.bad < 0) ? k : v.bad;
+    // U(k, :) right of k, W(k, :) from k to the left.
+    const double p0 = (!kSecond && at) ? r : m[0][0] * r, p1 = (kSecond && at) ? r : m[0][1] * r;
+    double* row = rows + k * kLeafLd;
+    row[lane] = p0;
+    row[lane + 32] = p1;
+    if (lane == 0) diag[k] = v.d * r;
+    v.d = fma(-u1, u1, v.b);
+    v.r = pivot_rsqrt(v.d);  // beside the row updates
+#pragma unroll
+    for (int i = 1; i <= ROWS; ++i) {
+      // U(k, row k + i); beyond the block: unused
+      const double u = i == 1 ? u1 : __shfl_sync(0xffffffffu, kSecond ? p1 : p0, l0 + q + i);
+      m[i - 1][0] = fma(-u, p0, (!kSecond && at) ? 0.0 : m[i][0]);  // column k becomes -U(k, row) W(k, k)
+      m[i - 1][1] = fma(-u, p1, (kSecond && at) ? 0.0 : m[i][1]);
+      if (i == 3) {
+        v.a = __shfl_sync(0xffffffffu, kSecond ? m[0][1] : m[0][0], l0 + q + 2);
+        v.b = __shfl_sync(0xffffffffu, kSecond ? m[1][1] : m[1][0], l0 + q + 2);
+      }
+    }
+    if (q & 1) {
+      __syncwarp();
+      __threadfence_block();
+      if (lane == 0) *done = k + 1;
+    }
+  }
+}
+
+template <bool kSecond>
+__device__ __forceinline__ void leaf_own_block(double (&m)[16][2], int blk, double* rows, double* diag,
+                                               volatile int* done, int* s_bad, int lane) {
+  const int l0 = (16 * blk) & 31;
+  LeafPivot v;
+  v.d = __shfl_sync(0xffffffffu, kSecond ? m[0][1] : m[0][0], l0);
+  v.a = __shfl_sync(0xffffffffu, kSecond ? m[0][1] : m[0][0], l0 + 1);
+  v.b = __shfl_sync(0xffffffffu, kSecond ? m[1][1] : m[1][0], l0 + 1);
+  v.r = pivot_rsqrt(v.d);
+  v.bad = -1;
+  leaf_own_steps<kSecond, 0, 15>(m, v, blk, rows, diag, done, lane);
+  leaf_own_steps<kSecond, 8, 7>(m, v, blk, rows, diag, done, lane);
+  if (v.bad >= 0 && lane == 0) atomicMin(s_bad, v.bad);
+}
+
+template <bool kSecond>
+__device__ __forceinline__ void leaf_follow_steps(double (&m)[16][2], int b, const double* rows, const volatile int* done,
+                                                  int warp, int lane) {
+#pragma unroll 1
+  for (int q = 0; q < 16; ++q) {
+    const int k = 16 * b + q;
+    if ((q & 1) == 0) {
+      // The owner never waits for this warp, so the wait ends; the count only keeps it bounded.
+      for (int spin = 0; *done < k + 2 && spin < (1 << 24); ++spin) {
+      }
+      __threadfence_block();
+    }
+    const bool at = lane == (k & 31);
+    const double* row = rows + k * kLeafLd;
+    const double p0 = row[lane], p1 = row[lane + 32];
+    double u[16];
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(row + 16 * warp + i);
+      u[i] = t.x;
+      u[i + 1] = t.y;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      m[i][0] = fma(-u[i], p0, (!kSecond && at) ? 0.0 : m[i][0]);
+      m[i][1] = fma(-u[i], p1, (kSecond && at) ? 0.0 : m[i][1]);
+    }
+  }
+}
 
 // Factor and invert the nb x nb (nb <= 64) diagonal block at (j0, j0) with the CTA's 128 threads: U in place in a,
 // X = U^-1 (upper; x's strict lower part is left as it is) into x.  Returns false (all threads) on a pivot that is
-// not > 0, after recording kStatusNotSPD with the global column (1-based).  The block is the kernel's critical path,
-// so it is factored by 8-column panels (three barriers per panel instead of two per column): the panel's 8 x 8
-// diagonal block by one warp with shuffles, its block row by a triangular solve per column, then the rank-8 update
-// of the trailing triangle with 8-deep dot products.  X is formed by blocks: the 8 x 8 diagonal blocks' inverses,
-// then joins of neighbouring blocks of 8, 16, 32.  The frame beyond nb is the identity.
+// not > 0, after recording kStatusNotSPD with the global column (1-based).  The frame beyond nb is the identity.
+//
+// The block is the kernel's critical path, and its chain of 64 pivots is what bounds it.  Factor and inverse come from
+// one elimination in registers (warp w holds rows 16 w .. 16 w + 15, lane l columns l and l + 32): with M = [A | I] the
+// step of pivot k scales row k by 1 / sqrt(M(k, k)) and subtracts U(k, i) times it from every row i > k.  Left of the
+// diagonal the rows then grow W = U^-T, which takes the place of A's lower triangle (at step k column k becomes
+// -U(k, i) W(k, k)), so the inverse costs no further step.  The owner warp runs down its 16 rows by shuffles alone,
+// leaving each final row in shared memory; the warps below follow it at their own pace (a row counter, no block
+// barrier).  One block alone (with its panel update): 39 k cycles, where panels of 8 columns with block barriers and a
+// separate block-wise inverse took 57 k; potrf + inverse n = 130 148 -> 118 us, 619 514 -> 420, 1788 1.41 -> 1.2 ms.
 // With a panel (the kp x nb block row U(j0 - kp : j0, j0 : j0 + nb), ld lda), the block's trailing update
-// A -= P^T P runs first, in shared memory with 8 x 4 register tiles per thread (gsm: the tile pipeline's region,
-// free while the leaf runs, holds P).
+// A -= P^T P runs first, by matrix instructions (gsm: the tile pipeline's region, free while the leaf runs, holds P).
 __device__ bool leaf_factor_invert(const double* panel, int kp, double* a, int lda, double* x, int ldx, int j0,
                                    int nb, DeviceStatus* st, double* smem, double* gsm) {
-  constexpr int P = 8;
-  double(*U)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(smem);
-  double(*X)[NB + 1] = U + NB;
-  double* dinv = reinterpret_cast<double*>(X + NB);
-  int* s_bad = reinterpret_cast<int*>(dinv + NB);
-  const int tid = threadIdx.x, lane = tid & 31;
+  double* rows = smem;                      // [64][kLeafLd]
+  double* diag = rows + NB * kLeafLd;       // U(k, k)
+  int* s_bad = reinterpret_cast<int*>(diag + NB);
+  volatile int* done = s_bad + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __syncthreads();
-  constexpr int kPer = NB * NB / kThreads / 2;
-  for (int pass = 0; pass < 2; ++pass) {
-    double v[kPer];
+  // Stage A (rows of the upper triangle) and P, coalesced, every load of a thread in flight at once.
+  constexpr int kPer = 32;
+  for (int base = 0; base < NB * NB; base += kThreads * kPer) {
+    double v[kPer], w[kPer];
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
-      const int idx = tid + kThreads * (pass * kPer + t), r = idx % NB, c = idx / NB;
+      const int idx = base + tid + kThreads * t, r = idx % NB, c = idx / NB;
       v[t] = c < nb ? (r <= c ? a[(j0 + r) + (size_t)(j0 + c) * lda] : 0.0) : (r == c ? 1.0 : 0.0);
+      w[t] = (panel && r < kp && c < nb) ? panel[r + (size_t)c * lda] : 0.0;
     }
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
-      const int idx = tid + kThreads * (pass * kPer + t), r = idx % NB, c = idx / NB;
-      U[r][c] = v[t];
+      const int idx = base + tid + kThreads * t, r = idx % NB, c = idx / NB;
+      rows[r * kLeafLd + c] = v[t];
+      if (panel) gsm[r * kLeafLd + c] = w[t];
     }
   }
-  if (tid == 0) *s_bad = -1;
+  if (tid == 0) { *s_bad = NB; *done = 0; }
+  __syncthreads();
   if (panel) {
-    double(*Pn)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(gsm);
-    for (int pass = 0; pass < 2; ++pass) {
-      double v[kPer];
+    // A -= P^T P on the upper 8 x 8 tiles with the FP64 matrix instruction: warp w takes tile rows w and 7 - w, nine
+    // tiles; lane l holds P(4 kk + l % 4, 8 t + l / 4) of either operand.
+    const int kr = lane & 3, cr = lane >> 2;
+    double acc[9][2];
 #pragma unroll
-      for (int t = 0; t < kPer; ++t) {
-        const int idx = tid + kThreads * (pass * kPer + t), r = idx % NB, c = idx / NB;
-        v[t] = (r < kp && c < nb) ? panel[r + (size_t)c * lda] : 0.0;
-      }
+    for (int t = 0; t < 9; ++t) acc[t][0] = acc[t][1] = 0.0;
+    const int rows0 = warp, rows1 = 7 - warp;  // tiles (rows0, rows0 .. 7), then (rows1, rows1 .. 7)
+#pragma unroll 4
+    for (int kk = 0; kk < NB; kk += 4) {       // rows of P beyond kp are zero
+      const double* pk = gsm + (kk + kr) * kLeafLd + cr;
+      const double a0 = pk[8 * rows0], a1 = pk[8 * rows1];
 #pragma unroll
-      for (int t = 0; t < kPer; ++t) {
-        const int idx = tid + kThreads * (pass * kPer + t);
-        Pn[idx % NB][idx / NB] = v[t];
+      for (int t = 0; t < 9; ++t) {
+        const bool first = t < 8 - rows0;
+        const double bf = pk[8 * (first ? rows0 + t : rows1 + t - (8 - rows0))];
+        tile::mma_f64(acc[t], first ? a0 : a1, bf);
       }
+    }
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      const bool first = t < 8 - rows0;
+      const int r = 8 * (first ? rows0 : rows1) + cr, c = 8 * (first ? rows0 + t : rows1 + t - (8 - rows0)) + 2 * kr;
+      double2* dst = reinterpret_cast<double2*>(rows + r * kLeafLd + c);
+      double2 v = *dst;
+      v.x -= acc[t][0];
+      v.y -= acc[t][1];
+      *dst = v;
     }
     __syncthreads();
-    // Thread (rb, cb) owns rows rb + 8 i and columns cb + 16 j (i < 8, j < 4): the 8 lanes of a row group read
-    // consecutive panel entries, the column reads are broadcasts.
-    const int rb = tid & 7, cb = tid >> 3;
-    double acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    for (int k = 0; k < kp; ++k) {
-      double pr[8], pc[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) pr[i] = Pn[k][rb + 8 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pc[j] = Pn[k][cb + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(pr[i], pc[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = rb + 8 * i, c = cb + 16 * j;
-        if (r <= c && c < nb) U[r][c] -= acc[i][j];
-      }
   }
-  const int tx = tid & 15, ty = tid >> 4;
-  for (int p0 = 0; p0 < NB; p0 += P) {
-    __syncthreads();
-    // (a) the 8 x 8 diagonal block by one warp: lane c (mod 8) holds its column.
-    if (tid < 32) {
-      const int c = lane & 7;
-      double d[P];
+  double m[16][2];
 #pragma unroll
-      for (int i = 0; i < P; ++i) d[i] = i <= c ? U[p0 + i][p0 + c] : 0.0;
-      int bad = -1;
-      double dv = 0.0;
+  for (int i = 0; i < 16; ++i)
 #pragma unroll
-      for (int k = 0; k < P; ++k) {
-        const double piv = __shfl_sync(0xffffffffu, d[k], k, P);
-        if (!(piv > 0.0) && bad < 0) bad = k;
-        const double inv = rsqrt(piv);
-        const double ukc = d[k] * inv;
-        if (c == k) dv = inv;
-#pragma unroll
-        for (int i = k + 1; i < P; ++i) {
-          const double uki = __shfl_sync(0xffffffffu, ukc, i, P);
-          if (i <= c) d[i] = fma(-uki, ukc, d[i]);
-        }
-        d[k] = ukc;
-      }
-      if (lane < P) {
-#pragma unroll
-        for (int i = 0; i < P; ++i)
-          if (i <= c) U[p0 + i][p0 + c] = d[i];
-        dinv[p0 + c] = dv;
-        if (lane == 0 && bad >= 0) *s_bad = p0 + bad;
-      }
-    }
-    __syncthreads();
-    if (*s_bad >= 0) {
-      if (tid == 0) set_status(st, kStatusNotSPD, j0 + *s_bad + 1, 0);
-      __syncthreads();
-      return false;
-    }
-    // (b) the panel's block row: U(p0:p0+8, c) = U_d^-T A(p0:p0+8, c), one thread per column.
-    {
-      const int c = p0 + P + tid;
-      if (c < NB) {
-        double u[P];
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          double s = U[p0 + q][c];
-#pragma unroll
-          for (int pp = 0; pp < q; ++pp) s = fma(-U[p0 + pp][p0 + q], u[pp], s);
-          u[q] = s * dinv[p0 + q];
-        }
-#pragma unroll
-        for (int q = 0; q < P; ++q) U[p0 + q][c] = u[q];
-      }
-    }
-    __syncthreads();
-    // (c) trailing update A(r, c) -= sum_q U(p0+q, r) U(p0+q, c), r <= c in [p0+8, 64).
-    {
-      const int b = p0 + P;
-      double uc[4][P];
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const int c = b + tx + 16 * jj;
-#pragma unroll
-        for (int q = 0; q < P; ++q) uc[jj][q] = c < NB ? U[p0 + q][c] : 0.0;
-      }
-      for (int i = 0; i < 8; ++i) {
-        const int r = b + ty + 8 * i;
-        if (r >= NB) break;
-        double ur[P];
-#pragma unroll
-        for (int q = 0; q < P; ++q) ur[q] = U[p0 + q][r];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const int c = b + tx + 16 * jj;
-          if (c >= r && c < NB) {
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int q = 0; q < P; q += 2) {
-              s0 = fma(ur[q], uc[jj][q], s0);
-              s1 = fma(ur[q + 1], uc[jj][q + 1], s1);
-            }
-            U[r][c] -= s0 + s1;
-          }
-        }
-      }
-    }
+    for (int j = 0; j < 2; ++j) m[i][j] = rows[(16 * warp + i) * kLeafLd + lane + 32 * j];
+  __syncthreads();  // every row has been read before the first final row is written
+#pragma unroll 1
+  for (int b = 0; b < warp; ++b) {
+    if (b < 2) leaf_follow_steps<false>(m, b, rows, done, warp, lane);
+    else leaf_follow_steps<true>(m, b, rows, done, warp, lane);
   }
+  if (warp < 2) leaf_own_block<false>(m, warp, rows, diag, done, s_bad, lane);
+  else leaf_own_block<true>(m, warp, rows, diag, done, s_bad, lane);
   __syncthreads();
-  // X = U^-1 by blocks, on every thread: the eight 8 x 8 diagonal blocks by back substitution (one thread per
-  // column), then neighbouring blocks of s = 8, 16, 32 are joined, X12 = -X11 (U12 X22): T = U12 X22 is written
-  // where X12 goes, then each thread forms its entries of -X11 T in registers before any of them is written back.
-  // (A back substitution per column over the whole block ran its last column's ~1800 dependent FMAs on one thread.)
-  for (int idx = tid; idx < NB * (NB + 1); idx += kThreads) (&X[0][0])[idx] = 0.0;
-  __syncthreads();
-  if (tid < NB) {
-    const int c = tid, p0 = (c / P) * P;
-    double xv[P];
-#pragma unroll
-    for (int ii = P - 1; ii >= 0; --ii) {
-      const int r = p0 + ii;
-      double t = 0.0;
-#pragma unroll
-      for (int jj = ii + 1; jj < P; ++jj) t = fma(U[r][p0 + jj], xv[jj], t);
-      xv[ii] = r > c ? 0.0 : (r == c ? dinv[c] : -dinv[r] * t);
-    }
-#pragma unroll
-    for (int ii = 0; ii < P; ++ii) X[p0 + ii][c] = xv[ii];
+  if (*s_bad < NB) {
+    if (tid == 0) set_status(st, kStatusNotSPD, j0 + *s_bad + 1, 0);
+    __syncthreads();
+    return false;
   }
-  // Each join has NB / 2 rows (pairs x rows of X12): thread (row = tid % 32, group = tid / 32) owns that row's
-  // columns group, group + 4, ..., so one load of the row's entry feeds up to eight independent sums.
-  constexpr int kCols = NB / 2 / 4;  // columns of X12 per thread at the widest join
-  const int jrow = tid % (NB / 2), jgrp = tid / (NB / 2);
-  for (int sz = P; sz < NB; sz *= 2) {
-    const int o = (jrow / sz) * 2 * sz, r = jrow % sz, c0 = o + sz, ncol = sz / 4;
-    __syncthreads();
-    // T = U12 X22 (X22 upper: T(r, c) sums q <= c), written where X12 goes.
-    double acc[kCols];
-#pragma unroll
-    for (int m = 0; m < kCols; ++m) acc[m] = 0.0;
-    for (int q = 0; q < sz; ++q) {
-      const double u = U[o + r][c0 + q];
-#pragma unroll
-      for (int m = 0; m < kCols; ++m) {
-        const int c = jgrp + 4 * m;
-        if (m < ncol && q <= c) acc[m] = fma(u, X[c0 + q][c0 + c], acc[m]);
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < kCols; ++m)
-      if (m < ncol) X[o + r][c0 + jgrp + 4 * m] = acc[m];
-    __syncthreads();
-    // X12 = -X11 T (X11 upper: row r sums q >= r); every entry is formed before any is written back.
-#pragma unroll
-    for (int m = 0; m < kCols; ++m) acc[m] = 0.0;
-    for (int q = r; q < sz; ++q) {
-      const double xr = X[o + r][o + q];
-#pragma unroll
-      for (int m = 0; m < kCols; ++m)
-        if (m < ncol) acc[m] = fma(xr, X[o + q][c0 + jgrp + 4 * m], acc[m]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int m = 0; m < kCols; ++m)
-      if (m < ncol) X[o + r][c0 + jgrp + 4 * m] = -acc[m];
-  }
-  __syncthreads();
+#pragma unroll 8
   for (int idx = tid; idx < NB * NB; idx += kThreads) {
     const int r = idx % NB, c = idx / NB;
     if (r <= c && c < nb) {
-      a[(j0 + r) + (size_t)(j0 + c) * lda] = U[r][c];
-      x[(j0 + r) + (size_t)(j0 + c) * ldx] = X[r][c];
+      a[(j0 + r) + (size_t)(j0 + c) * lda] = r == c ? diag[r] : rows[r * kLeafLd + c];
+      x[(j0 + r) + (size_t)(j0 + c) * ldx] = rows[c * kLeafLd + r];  // X(r, c) = W(c, r)
     }
   }
   __syncthreads();
   return true;
 }
-
 
 __device__ __forceinline__ GemmDesc<double> tile_desc(int M, int N, int K, double alpha, const double* A, int lda,
                                                       int transA, const double* B, int ldb, double beta, double* C,
@@ -371,7 +351,11 @@ __global__ void __launch_bounds__(kThreads, 1) potrf_persistent_kernel(PotrfPara
           rem -= cnt;
         }
         const int p0 = pr * 2 * sz, s2 = min(sz, n - p0 - sz);
-        const int rb = rem % tb, cb = rem / tb;
+        // Long sums first (K grows with the column block in the first product, shrinks with the row block in the
+        // second), so that a CTA's second tile is a short one: at n = 1788 the top level's 196 tiles take 148 CTAs 1.3
+        // instead of 2 longest tiles' time per product.
+        const int ncb = (s2 + NB - 1) / NB;
+        const int rb = phase == 0 ? rem % tb : rem / ncb, cb = phase == 0 ? ncb - 1 - rem / tb : rem % ncb;
         const int r0 = p0 + rb * NB, c0 = p0 + sz + cb * NB;
         const int rows = NB, cols = min(NB, p0 + sz + s2 - c0);
         double* tt = p.t + r0 + (size_t)c0 * n;
