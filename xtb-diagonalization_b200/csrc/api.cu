@@ -57,7 +57,7 @@ std::atomic<long> g_band_width{32};   // band width of the two-stage reduction (
 std::atomic<long> g_autotune{0};      // 1: solves use the autotuned plan nearest their size (xtb_gpu_autotune)
 std::atomic<long> g_batch_grid{1};    // 1: batch workers size each resident reduction's grid to its matrix
 std::atomic<long> g_dgemm_engine{1};  // FP64 GEMMs: 0 DMMA, 1 Ozaki (int8 tcgen05) where eligible, 2 Ozaki always
-std::atomic<long> g_dc_leaf{16};      // divide and conquer: subtrees of at most this size solved directly (0: none)
+std::atomic<long> g_dc_leaf{16};      // divide and conquer: nonzero: subtrees of at most 64 on one CTA each (0: none)
 std::atomic<long> g_backtransform{1};  // 1: C = (X Q) Z with X Q formed beside the tridiagonal eigensolve (n >= 512)
 std::atomic<long> g_sytrd_tail{64};  // the resident reduction's last columns (at most this many) on one CTA (0: off)
 std::atomic<long> g_test_stall{0};    // failure-detection test hook: 1 makes the resident reduction's barriers unreachable
@@ -74,7 +74,7 @@ struct Plan {
   int dgemm = 0;       // FP64 GEMM engine of the large GEMMs: 0 DMMA, 1 or 2 int8 Ozaki
   int batch_grid = 0;  // 1: a batch worker's solve, its resident reduction sized to its matrix (sytrd_grid 0)
   int xq = 1;          // generalized one-stage solves with n >= kXqMinN: C = (X Q) Z, X Q formed beside the D&C
-  int leaf = 16;       // divide and conquer leaf size (0: 1 x 1 leaves; 16, 32, 64: direct solves of the subtrees)
+  int leaf = 16;       // divide and conquer: nonzero: subtrees of at most 64 on one CTA each (0: 1 x 1 leaves)
   int tail = 64;       // the reduction's trailing block of at most this order finished on one CTA (0: none)
   double ms = 0.0;     // measured time of the tuned plan
   long long sig() const {
@@ -1606,10 +1606,10 @@ int xtb_gpu_autotune(int n, int precision, void* stream) {
     consider(p);
   }
   {
-    // The divide and conquer's leaf size: 1 x 1 leaves, or direct solves of the subtrees of at most 16 / 32 / 64.
+    // The divide and conquer's leaves: 1 x 1, or subtrees of at most 64 on one CTA each (16, 32 and 64 alike).
     const Plan r = best;
-    for (int leaf : {0, 16, 32, 64}) {
-      if (leaf == r.leaf) continue;
+    for (int leaf : {0, 16}) {
+      if ((leaf != 0) == (r.leaf != 0)) continue;
       Plan p = r;
       p.leaf = leaf;
       consider(p);

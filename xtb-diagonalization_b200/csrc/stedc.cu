@@ -3,7 +3,8 @@
 // merge is Stages/ParallelDivideAndConquer.swift:42-211, a port of LAPACK's dlaed1/2/3).
 //
 // B200 design.  The recursion is flattened into levels: the tree of tears is fixed by n alone, so every merge of one
-// level runs in the same launches (one CTA or warp per merge / root / column), bottom-up from 1 x 1 leaves.  Per level:
+// level runs in the same launches (one CTA or warp per merge / root / column).  The subtrees of at most 64 are solved by
+// one CTA each in shared memory (dc_subtree_kernel); the levels above them run bottom-up.  Per level:
 //   deflate   one CTA per merge: z from the halves' boundary rows, merge-sort of the two ascending eigenvalue lists,
 //             small-z deflation (rho |z_i| <= tol) and close-pair deflation by Givens rotation (Dongarra-Sorensen),
 //             classification of the surviving columns (upper half only / both / lower half only) so the merge GEMM
@@ -127,151 +128,6 @@ __global__ void dc_identity_kernel(int n, int ld, double* q, double* qb, const d
     qb[i + (size_t)j * ld] = v;
     if (j == 0) dnext[i] = dd[i];
   }
-}
-
-// ------------------------------------------------------------------------------------------------ leaves
-
-constexpr int kLeafMax = 64;
-
-// Leaf blocks: the subtrees of the tear tree at depth `depth` (every one of them at most kLeafMax long), each solved
-// directly by one CTA instead of by the merge levels below it.  Block i is found by walking the tree's halving from
-// the root along the bits of i (most significant first), the same split as build_levels: [a, b) -> [a, a + (b-a)/2),
-// [a + (b-a)/2, b).  The block's tridiagonal is the scaled one with the tears of its two ends only (its inner splits
-// are not torn because no merge undoes them); cyclic Jacobi with a round-robin ordering (m/2 disjoint rotations per
-// round) diagonalises it in shared memory, and its eigenvalues (ascending) and eigenvectors become the block's entry
-// state of the first merge level: dd / dnext and the diagonal block of both eigenvector buffers.
-__global__ void __launch_bounds__(256) dc_leaf_kernel(int n, int depth, const double* __restrict__ d,
-                                                      const double* __restrict__ ee, const double* __restrict__ scale,
-                                                      double* dd, double* dnext, double* qa, double* qb, int ld) {
-  extern __shared__ __align__(16) unsigned char leaf_smem[];  // a and v, kLeafMax x (kLeafMax + 1) each
-  double(*a)[kLeafMax + 1] = reinterpret_cast<double(*)[kLeafMax + 1]>(leaf_smem);
-  double(*v)[kLeafMax + 1] = a + kLeafMax;
-  __shared__ double red[32];
-  __shared__ double rot_c[kLeafMax / 2], rot_s[kLeafMax / 2];
-  __shared__ int rot_p[kLeafMax / 2], rot_q[kLeafMax / 2];
-  __shared__ int perm[kLeafMax];
-  int lo = 0, hi = n;
-  for (int l = depth - 1; l >= 0; --l) {
-    const int mid = lo + (hi - lo) / 2;
-    if ((blockIdx.x >> l) & 1) lo = mid;
-    else hi = mid;
-  }
-  const int m = hi - lo;
-  if (m <= 0 || m > kLeafMax) return;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const double sc = scale[0];
-  const double inv = sc > 0.0 ? 1.0 / sc : 1.0;
-  for (int t = tid; t < m * m; t += nt) {
-    const int r = t % m, c = t / m;
-    double x = 0.0;
-    if (r == c) {
-      x = d[lo + r] * inv;
-      if (r == 0 && lo > 0) x -= fabs(ee[lo - 1]);
-      if (r == m - 1 && hi < n) x -= fabs(ee[hi - 1]);
-    } else if (r == c + 1 || c == r + 1) {
-      x = ee[lo + min(r, c)];
-    }
-    a[r][c] = x;
-    v[r][c] = r == c ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  const int kp = (m + 1) & ~1;
-  // Converged once the off-diagonal mass is below 1e-28 of the diagonal's: rotations leave about m eps^2 of it in
-  // rounding (3e-30 at m = 64), so the test sits a little above that floor; the eigenvalues' error is quadratic in
-  // it and the residual linear (about 1e-14 relative).
-  for (int sweep = 0; sweep < 15 && m > 1; ++sweep) {
-    double off = 0.0, dg = 0.0;
-    for (int t = tid; t < m * m; t += nt) {
-      const int r = t % m, c = t / m;
-      if (r != c) off += a[r][c] * a[r][c];
-      else dg += a[r][c] * a[r][c];
-    }
-    off = block_sum(off, red);
-    dg = block_sum(dg, red);
-    if (off <= 1e-28 * dg || off == 0.0) break;
-    for (int round = 0; round < kp - 1; ++round) {
-      if (tid < kp / 2) {
-        auto at = [&](int pos) { return pos == 0 ? 0 : 1 + (round + pos - 1) % (kp - 1); };
-        int p = at(tid), q = at(kp - 1 - tid);
-        if (p > q) { const int x = p; p = q; q = x; }
-        double c = 1.0, sn = 0.0;
-        if (q < m) {
-          const double apq = a[p][q];
-          if (apq != 0.0) {
-            const double tau = (a[q][q] - a[p][p]) / (2.0 * apq);
-            double t;
-            if (fabs(tau) > 1e150) t = 0.5 / tau;
-            else t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-            c = rsqrt(1.0 + t * t);
-            sn = t * c;
-          }
-        }
-        rot_p[tid] = p;
-        rot_q[tid] = q;
-        rot_c[tid] = c;
-        rot_s[tid] = sn;
-      }
-      __syncthreads();
-      for (int t = tid; t < (kp / 2) * m; t += nt) {  // rows p, q of a
-        const int r = t / m, j = t % m;
-        const int p = rot_p[r], q = rot_q[r];
-        if (q >= m) continue;
-        const double c = rot_c[r], sn = rot_s[r];
-        const double xp = a[p][j], xq = a[q][j];
-        a[p][j] = c * xp - sn * xq;
-        a[q][j] = sn * xp + c * xq;
-      }
-      __syncthreads();
-      for (int t = tid; t < (kp / 2) * m; t += nt) {  // columns p, q of a and of v
-        const int r = t / m, i = t % m;
-        const int p = rot_p[r], q = rot_q[r];
-        if (q >= m) continue;
-        const double c = rot_c[r], sn = rot_s[r];
-        double xp = a[i][p], xq = a[i][q];
-        a[i][p] = c * xp - sn * xq;
-        a[i][q] = sn * xp + c * xq;
-        xp = v[i][p];
-        xq = v[i][q];
-        v[i][p] = c * xp - sn * xq;
-        v[i][q] = sn * xp + c * xq;
-      }
-      __syncthreads();
-    }
-  }
-  // ascending order of the eigenvalues (ties by index)
-  if (tid < m) {
-    const double di = a[tid][tid];
-    int r = 0;
-    for (int j = 0; j < m; ++j) {
-      const double dj = a[j][j];
-      r += (okey(dj) < okey(di) || (okey(dj) == okey(di) && j < tid)) ? 1 : 0;
-    }
-    perm[r] = tid;
-  }
-  __syncthreads();
-  if (tid < m) {
-    const double lam = a[perm[tid]][perm[tid]];
-    dd[lo + tid] = lam;
-    dnext[lo + tid] = lam;
-  }
-  for (int t = tid; t < m * m; t += nt) {
-    const int r = t % m, c = t / m;
-    const double x = v[r][perm[c]];
-    qa[(size_t)(lo + r) + (size_t)(lo + c) * ld] = x;
-    qb[(size_t)(lo + r) + (size_t)(lo + c) * ld] = x;
-  }
-}
-
-// Depth of the leaf blocks for leaves of at most `leaf` (0 or 1: the tree goes down to 1 x 1 leaves, no leaf solve):
-// the first depth at which the largest block (the larger half, repeatedly) is at most `leaf`.
-int leaf_depth(int n, int leaf) {
-  if (leaf <= 1) return -1;
-  int d = 0, mx = n;
-  while (mx > leaf) {
-    mx = mx - mx / 2;
-    ++d;
-  }
-  return d;
 }
 
 // Block-wide exclusive scan of one int per thread; returns the exclusive prefix, *total receives the sum.
@@ -533,15 +389,47 @@ __global__ void dc_gather_kernel(DcBufs B) {
 
 // ------------------------------------------------------------------------------------------------ secular equation
 
+// 1 / x and a / x without a branch, so that the divisions of a loop overlap (the compiler's division branches to a slow
+// path, which left every one's latency of about 150 cycles exposed: a thread's 13 poles took 2300 cycles per evaluation).
+// The hardware's approximation, one third-order Newton step, y (1 + h + h^2) with h = 1 - x y, and for the quotient
+// Markstein's residual correction (IA-64 and Elementary Functions, 2000); either rounds once at the end.  x is normal: the
+// differences here are at least about 1e-31 of the scaled spectrum, and other values give a NaN, as bad input does.
+__device__ __forceinline__ double rcp_normal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = fma(-x, y, 1.0);
+  return fma(y, fma(h, h, h), y);
+}
+__device__ __forceinline__ double div_normal(double a, double x) {
+  const double y = rcp_normal(x), q = a * y;
+  return fma(fma(-q, x, a), y, q);
+}
+
+// Sums over the poles left of the root (psi <= 0), right of it (phi >= 0) and their derivatives; the sum of the terms'
+// absolute values is phi - psi.
 struct SecSums {
-  double psi, dpsi, phi, dphi, asum;
+  double psi, dpsi, phi, dphi;
 };
 
-// A root is solved by WPR warps together (one CTA of 32 WPR threads when WPR > 1): every sum runs over the poles
+// Threads per root: WPR warps, or eight lanes (WPR 0).
+template <int WPR>
+constexpr int kRootThreads = WPR == 0 ? 8 : 32 * WPR;
+
+// A root is solved by WPR warps together (one CTA of 32 WPR threads when WPR > 1) or by eight lanes: every sum runs over the poles
 // strided by the group's threads, then across its warps in warp order through shared memory (sh: 2 x 5 x WPR doubles,
-// alternating by `tog`, so one __syncthreads per sum; every thread receives the same value).
+// alternating by `tog`, so one __syncthreads per sum; every thread receives the same value).  The groups of eight of a warp may diverge.
 template <int WPR>
 __device__ __forceinline__ void group_sums(double* v, int cnt, double* sh, int& tog) {
+  if constexpr (WPR == 0) {
+    const unsigned mask = 0xffu << (threadIdx.x & 24);
+#pragma unroll 5
+    for (int j = 0; j < cnt; ++j) {
+      v[j] += __shfl_xor_sync(mask, v[j], 4);
+      v[j] += __shfl_xor_sync(mask, v[j], 2);
+      v[j] += __shfl_xor_sync(mask, v[j], 1);
+    }
+    return;
+  }
 #pragma unroll 5
   for (int j = 0; j < cnt; ++j) v[j] = warp_sum(v[j]);
   if constexpr (WPR > 1) {
@@ -563,19 +451,23 @@ __device__ __forceinline__ void group_sums(double* v, int cnt, double* sh, int& 
 template <int WPR>
 __device__ __forceinline__ SecSums sec_eval(const double* dl, const double* z, int K, int o, int a, double tau,
                                             double* sh, int& tog) {
-  const int lane = threadIdx.x & (32 * WPR - 1);
-  SecSums r{0, 0, 0, 0, 0};
+  const int lane = threadIdx.x & (kRootThreads<WPR> - 1);
+  SecSums r{0, 0, 0, 0};
   const double dlo = dl[o];
-  for (int i = lane; i < K; i += 32 * WPR) {
+#pragma unroll 4
+  for (int i = lane; i < K; i += kRootThreads<WPR>) {
     const double del = (dl[i] - dlo) - tau;
-    const double inv = 1.0 / del;
-    const double t = z[i] * z[i] * inv;
-    if (i <= a) { r.psi += t; r.dpsi += t * inv; } else { r.phi += t; r.dphi += t * inv; }
-    r.asum += fabs(t);
+    const double inv = rcp_normal(del);
+    const double t = z[i] * z[i] * inv, dt = t * inv;
+    const bool left = i <= a;
+    r.psi += left ? t : 0.0;
+    r.dpsi += left ? dt : 0.0;
+    r.phi += left ? 0.0 : t;
+    r.dphi += left ? 0.0 : dt;
   }
-  double v[5] = {r.psi, r.dpsi, r.phi, r.dphi, r.asum};
-  group_sums<WPR>(v, 5, sh, tog);
-  return SecSums{v[0], v[1], v[2], v[3], v[4]};
+  double v[4] = {r.psi, r.dpsi, r.phi, r.dphi};
+  group_sums<WPR>(v, 4, sh, tog);
+  return SecSums{v[0], v[1], v[2], v[3]};
 }
 
 // Root j of 1/rho + sum_i z_i^2 / (dl_i - lambda) = 0 (rho > 0, dl ascending): lambda = dl[o] + tau.
@@ -583,7 +475,7 @@ __device__ __forceinline__ SecSums sec_eval(const double* dl, const double* z, i
 template <int WPR>
 __device__ bool secular_root(const double* dl, const double* z, int K, double rho, int j, int* o_out,
                              double* tau_out, double* sh) {
-  const int lane = threadIdx.x & (32 * WPR - 1);
+  const int lane = threadIdx.x & (kRootThreads<WPR> - 1);
   int tog = 0;
   const double rinv = 1.0 / rho;
   if (K == 1) {
@@ -592,35 +484,37 @@ __device__ bool secular_root(const double* dl, const double* z, int K, double rh
     return true;
   }
   int o, a;
-  double lo, hi;
+  double lo, hi, tau;
+  SecSums S{0, 0, 0, 0};
+  // The evaluation at the middle of the interval chooses the origin (the nearer pole) and is the first iterate.
+  bool have = false;
   if (j < K - 1) {
-    const double dj = dl[j], gap = dl[j + 1] - dj;
-    double fm = 0.0;
-    for (int i = lane; i < K; i += 32 * WPR) fm += z[i] * z[i] / ((dl[i] - dj) - 0.5 * gap);
-    group_sums<WPR>(&fm, 1, sh, tog);
-    fm = rinv + fm;
-    if (fm >= 0.0) { o = j; lo = 0.0; hi = 0.5 * gap; }
-    else { o = j + 1; lo = -0.5 * gap; hi = 0.0; }
+    const double gap = dl[j + 1] - dl[j];
     a = j;
+    S = sec_eval<WPR>(dl, z, K, j, a, 0.5 * gap, sh, tog);
+    have = true;
+    if (rinv + S.psi + S.phi >= 0.0) { o = j; lo = 0.0; hi = tau = 0.5 * gap; }
+    else { o = j + 1; lo = tau = -0.5 * gap; hi = 0.0; }
   } else {
     double zz = 0.0;
-    for (int i = lane; i < K; i += 32 * WPR) zz += z[i] * z[i];
+    for (int i = lane; i < K; i += kRootThreads<WPR>) zz += z[i] * z[i];
     group_sums<WPR>(&zz, 1, sh, tog);
     o = K - 1;
     lo = 0.0;
     hi = rho * zz;
     a = K - 2;
+    tau = 0.5 * (lo + hi);
   }
   const int b = a + 1;
   const double dlo = dl[o];
   const double pa = dl[a] - dlo, pb = dl[b] - dlo;  // poles relative to the origin
-  double tau = 0.5 * (lo + hi);
   bool conv = false;
   for (int it = 0; it < 120; ++it) {
-    const SecSums S = sec_eval<WPR>(dl, z, K, o, a, tau, sh, tog);
+    if (!have) S = sec_eval<WPR>(dl, z, K, o, a, tau, sh, tog);
     const double f = rinv + S.psi + S.phi;
-    const double errb = 8.0 * kEps * (rinv + S.asum) + kEps * fabs(tau) * (S.dpsi + S.dphi);
-    if (fabs(f) <= errb) { conv = true; break; }
+    const double errb = 8.0 * kEps * (rinv + (S.phi - S.psi)) + kEps * fabs(tau) * (S.dpsi + S.dphi);
+    if (!have && fabs(f) <= errb) { conv = true; break; }
+    have = false;
     if (f < 0.0) lo = tau; else hi = tau;
     if (hi - lo <= 2.0 * kEps * fmax(fabs(lo), fabs(hi))) { conv = true; break; }
     // Two-pole rational model c + A/(da - eta) + B/(db - eta) matching psi, psi', phi, phi' at tau.
@@ -630,15 +524,15 @@ __device__ bool secular_root(const double* dl, const double* z, int K, double rh
     const double bq = c * (da + db) + A + Bm, cq = da * db * f;
     double cand1 = NAN, cand2 = NAN;
     if (c == 0.0) {
-      if (bq != 0.0) cand1 = cq / bq;
+      if (bq != 0.0) cand1 = div_normal(cq, bq);
     } else {
       double disc = bq * bq - 4.0 * c * cq;
       if (disc < 0.0) disc = 0.0;
       const double sq = sqrt(disc);
       const double big = (bq >= 0.0) ? (bq + sq) : (bq - sq);
       if (big != 0.0) {
-        cand1 = big / (2.0 * c);
-        cand2 = 2.0 * cq / big;
+        cand1 = div_normal(big, 2.0 * c);
+        cand2 = div_normal(2.0 * cq, big);
       }
     }
     double tn = NAN;
@@ -728,9 +622,10 @@ __global__ void dc_zhat_kernel(DcBufs B) {
   const double* dl = B.dlam + s;
   const double di = dl[i];
   double prod = 1.0;
+#pragma unroll 4
   for (int j = lane; j < K; j += 32) {
     const double del = (di - dl[B.rorg[s + j]]) - B.rtau[s + j];
-    prod *= (j == i) ? -del : del / (di - dl[j]);
+    prod *= (j == i) ? -del : div_normal(del, j == i ? 1.0 : di - dl[j]);
   }
   prod = warp_prod(prod);
   if (lane == 0) {
@@ -760,13 +655,511 @@ __global__ void dc_vectors_kernel(DcBufs B) {
   const double* dl = B.dlam + s;
   const double dlo = dl[B.rorg[s + j]], tau = B.rtau[s + j];
   double ss = 0.0;
+#pragma unroll 4
   for (int i = lane; i < K; i += 32) {
-    const double u = B.zh[s + i] / ((dl[i] - dlo) - tau);
+    const double u = div_normal(B.zh[s + i], (dl[i] - dlo) - tau);
     ss += u * u;
   }
   ss = warp_sum(ss);
   const double inv = 1.0 / sqrt(ss);
-  for (int i = lane; i < K; i += 32) up[B.slotOf[s + i]] = (B.zh[s + i] / ((dl[i] - dlo) - tau)) * inv;
+#pragma unroll 4
+  for (int i = lane; i < K; i += 32) up[B.slotOf[s + i]] = div_normal(B.zh[s + i], (dl[i] - dlo) - tau) * inv;
+}
+
+// ------------------------------------------------------------------------------------------------ small subtrees
+
+constexpr int kSubMax = 64;    // largest subtree solved by one CTA
+constexpr int kSubLeaf = 8;    // its leaves, diagonalised by Jacobi, one warp each
+constexpr int kSubThreads = 512;  // eight lanes per position
+constexpr int kSubLd = kSubMax + 1;
+
+// Depth of the tree of halvings at which the largest block (the larger half, repeatedly) is at most `size`.
+__host__ __device__ inline int tree_depth(int n, int size) {
+  int d = 0;
+  while (n > size) {
+    n -= n / 2;
+    ++d;
+  }
+  return d;
+}
+// Block i at depth `depth` of the tree over [lo, hi): the bits of i choose the halves, most significant first, with the
+// split of build_levels.
+__host__ __device__ inline void tree_block(int i, int depth, int& lo, int& hi) {
+  for (int l = depth - 1; l >= 0; --l) {
+    const int mid = lo + (hi - lo) / 2;
+    if ((i >> l) & 1) lo = mid;
+    else hi = mid;
+  }
+}
+
+struct SubShared {
+  double q[2][kSubMax][kSubLd];  // eigenvectors of the current blocks, and those of the next level
+  double u[kSubMax][kSubLd];     // rank-one eigenvectors, row = survivor
+  double d[2][kSubMax];          // eigenvalues by position
+  double e[kSubMax];             // off-diagonal (scaled)
+  double sd[kSubMax], sz[kSubMax];                // sorted d and z of a merge
+  double dl[kSubMax], zk[kSubMax], zh[kSubMax];   // survivors' poles, z, recomputed z
+  double tau[kSubMax], lam[kSubMax], dv[kSubMax]; // roots, deflated values
+  double rc[kSubMax], rs[kSubMax];                // rotations
+  int perm[kSubMax], flag[kSubMax], nd[kSubMax], cand[kSubMax];
+  int col[kSubMax], dcol[kSubMax], org[kSubMax], out[kSubMax], ri[kSubMax], rj[kSubMax];
+  int K[4], nrot[4];
+  double rho[4];
+};
+
+// Jacobi on the warp's m x m leaf (m <= 8) at local position s: q holds the symmetric block on entry and its
+// eigenvectors on exit, d the eigenvalues (ascending).  a: the other q buffer, work space at the same place.
+// Round-robin ordering, m / 2 disjoint rotations per round; a rotation's angle from two reciprocal square roots,
+// cos 2t = |h| / r, sin 2t = b / r with h = a_qq - a_pp, b = 2 a_pq, r = |(h, b)|.
+__device__ __forceinline__ void sub_leaf(SubShared& S, double (*q)[kSubLd], double (*a)[kSubLd], double* d, int s, int m) {
+  const int lane = threadIdx.x & 31, vr = lane >> 2, vj = lane & 3;  // row vr, columns vj and vj + 4
+#pragma unroll
+  for (int h = 0; h < 8; h += 4) {
+    const int c = vj + h;
+    if (vr < m && c < m) {
+      a[s + vr][s + c] = q[s + vr][s + c];
+      q[s + vr][s + c] = vr == c ? 1.0 : 0.0;
+    }
+  }
+  __syncwarp();
+  const int kp = (m + 1) & ~1;
+  for (int sweep = 0; sweep < 15 && m > 1; ++sweep) {
+    double off = 0.0, dg = 0.0;
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+      const int c = vj + h;
+      const double x = (vr < m && c < m) ? a[s + vr][s + c] : 0.0;
+      if (vr != c) off = fma(x, x, off);
+      else dg = fma(x, x, dg);
+    }
+    off = warp_sum(off);
+    dg = warp_sum(dg);
+    // Rotations leave about m eps^2 of the diagonal's mass in rounding: 1e-28 is a little above that floor.
+    if (off <= 1e-28 * dg || off == 0.0) break;
+    for (int round = 0; round < kp - 1; ++round) {
+      // Lane i < kp / 2 forms rotation i; every lane gets the ones it needs by shuffle.
+      auto at = [&](int pos) {
+        const int x = round + pos - 1;
+        return pos == 0 ? 0 : 1 + (x >= kp - 1 ? x - (kp - 1) : x);
+      };
+      int p = 0, pq = 0;
+      double c = 1.0, sn = 0.0;
+      if (lane < kp / 2) {
+        p = at(lane);
+        pq = at(kp - 1 - lane);
+        if (p > pq) { const int x = p; p = pq; pq = x; }
+        if (pq < m) {
+          const double apq = a[s + p][s + pq];
+          const double h = a[s + pq][s + pq] - a[s + p][s + p], b = 2.0 * apq;
+          const double r2 = fma(h, h, b * b);
+          if (apq != 0.0 && r2 > 1e-290) {
+            const double ri = rsqrt(r2);
+            const double c2 = fma(0.5 * fabs(h), ri, 0.5);
+            const double rc = rsqrt(c2);
+            c = c2 * rc;
+            sn = copysign(0.5, h) * b * ri * rc;
+          }
+        }
+      }
+      // Two-sided update by 2 x 2 blocks: lane (i, j) = (lane / 4, lane % 4), pairs i and j, lanes 0 .. 15.
+      const int i = (lane >> 2) & 3, j = lane & 3;
+      const int pi = __shfl_sync(0xffffffffu, p, i), qi = __shfl_sync(0xffffffffu, pq, i);
+      const int pj = __shfl_sync(0xffffffffu, p, j), qj = __shfl_sync(0xffffffffu, pq, j);
+      const double ci = __shfl_sync(0xffffffffu, c, i), si = __shfl_sync(0xffffffffu, sn, i);
+      const double cj = __shfl_sync(0xffffffffu, c, j), sj = __shfl_sync(0xffffffffu, sn, j);
+      const bool on = lane < 16 && i < kp / 2 && j < kp / 2, qi_in = qi < m, qj_in = qj < m;
+      double xpp = 0.0, xpq = 0.0, xqp = 0.0, xqq = 0.0;
+      if (on) {
+        xpp = a[s + pi][s + pj];
+        if (qj_in) xpq = a[s + pi][s + qj];
+        if (qi_in) xqp = a[s + qi][s + pj];
+        if (qi_in && qj_in) xqq = a[s + qi][s + qj];
+      }
+      // The rotations of the vectors: columns p, q of q, one lane per (row, pair).
+      const int vp = __shfl_sync(0xffffffffu, p, vj), vq = __shfl_sync(0xffffffffu, pq, vj);
+      const double vc = __shfl_sync(0xffffffffu, c, vj), vs = __shfl_sync(0xffffffffu, sn, vj);
+      const bool von = vr < m && vj < kp / 2 && vq < m;
+      double vxp = 0.0, vxq = 0.0;
+      if (von) {
+        vxp = q[s + vr][s + vp];
+        vxq = q[s + vr][s + vq];
+      }
+      __syncwarp();
+      if (on) {
+        // rows: (p, q) <- (c p - s q, s p + c q), then columns alike
+        const double tpp = ci * xpp - si * xqp, tqp = si * xpp + ci * xqp;
+        const double tpq = ci * xpq - si * xqq, tqq = si * xpq + ci * xqq;
+        a[s + pi][s + pj] = cj * tpp - sj * tpq;
+        if (qj_in) a[s + pi][s + qj] = sj * tpp + cj * tpq;
+        if (qi_in) a[s + qi][s + pj] = cj * tqp - sj * tqq;
+        if (qi_in && qj_in) a[s + qi][s + qj] = sj * tqp + cj * tqq;
+      }
+      if (von) {
+        q[s + vr][s + vp] = vc * vxp - vs * vxq;
+        q[s + vr][s + vq] = vs * vxp + vc * vxq;
+      }
+      __syncwarp();
+    }
+  }
+  // Ascending order (ties by index); the columns of q move through registers.
+  double w = 0.0;
+  int rank = 0;
+  if (lane < m) {
+    w = a[s + lane][s + lane];
+    for (int t = 0; t < m; ++t) {
+      const double o = a[s + t][s + t];
+      rank += (okey(o) < okey(w) || (okey(o) == okey(w) && t < lane)) ? 1 : 0;
+    }
+  }
+  double v[2] = {0.0, 0.0};
+  int to[2] = {0, 0};
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c = vj + 4 * h;
+    to[h] = __shfl_sync(0xffffffffu, rank, c);
+    if (vr < m && c < m) v[h] = q[s + vr][s + c];
+  }
+  __syncwarp();
+  if (lane < m) d[s + rank] = w;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (vr < m && vj + 4 * h < m) q[s + vr][s + to[h]] = v[h];
+  // the work block is the next level's output buffer: zero outside what the merges write
+#pragma unroll
+  for (int h = 0; h < 8; h += 4)
+    if (vr < m && vj + h < m) a[s + vr][s + vj + h] = 0.0;
+  __syncwarp();
+}
+
+// Deflation of one merge (n <= 64) by one warp: the steps of dc_deflate_kernel on two positions per lane.
+__device__ __forceinline__ void sub_deflate(SubShared& S, int mi, int s, int n, double dmax) {
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+  double* sd = S.sd + s;
+  double* sz = S.sz + s;
+  int* flag = S.flag + s;  // 1: deflated
+  const double rho = S.rho[mi];
+  double zmax = 0.0;
+  for (int p = lane; p < n; p += 32) zmax = fmax(zmax, fabs(sz[p]));
+  zmax = warp_max(zmax);
+  const double tol = 8.0 * kEps * fmax(dmax, zmax);
+  // Small-z deflation; the positions kept, in order.
+  int mk = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int p = lane + 32 * h;
+    const bool keep = p < n && rho * fabs(sz[p]) > tol;
+    if (p < n) flag[p] = keep ? 0 : 1;
+    const unsigned b = __ballot_sync(full, keep);
+    if (keep) S.nd[s + mk + __popc(b & below)] = p;
+    mk += __popc(b);
+  }
+  __syncwarp();
+  // Pairs that pass the close-pair test before any rotation, then the sequential chain over them.
+  int nc = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = lane + 32 * h;
+    bool close = false;
+    if (i < mk - 1) {
+      const int a = S.nd[s + i], b = S.nd[s + i + 1];
+      const double za = sz[a], zb = sz[b], t = hypot(za, zb);
+      close = fabs((sd[b] - sd[a]) * (zb / t) * (-za / t)) <= tol;
+    }
+    const unsigned b = __ballot_sync(full, close);
+    if (close) S.cand[s + nc + __popc(b & below)] = i;
+    nc += __popc(b);
+  }
+  __syncwarp();
+  int nrot = 0;
+  if (lane == 0) {
+    int next = 0;
+    for (int c = 0; c < nc; ++c) {
+      int i = S.cand[s + c];
+      if (i < next) continue;
+      for (; i < mk - 1; ++i) {
+        const int a = S.nd[s + i], b = S.nd[s + i + 1];
+        const double za = sz[a], zb = sz[b], t = hypot(za, zb);
+        const double cs = zb / t, sn = -za / t, da = sd[a], db = sd[b];
+        if (!(fabs((db - da) * cs * sn) <= tol)) break;
+        sz[b] = t;
+        sz[a] = 0.0;
+        sd[a] = da * cs * cs + db * sn * sn;
+        sd[b] = da * sn * sn + db * cs * cs;
+        flag[a] = 1;
+        S.ri[s + nrot] = S.perm[s + a];
+        S.rj[s + nrot] = S.perm[s + b];
+        S.rc[s + nrot] = cs;
+        S.rs[s + nrot] = sn;
+        ++nrot;
+      }
+      next = i + 1;
+    }
+    S.nrot[mi] = nrot;
+  }
+  __syncwarp();
+  int K = 0, nd = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int p = lane + 32 * h;
+    const bool in = p < n, gone = in && flag[p] != 0;
+    const unsigned bs = __ballot_sync(full, in && !gone), bd = __ballot_sync(full, gone);
+    if (in && !gone) {
+      const int i = K + __popc(bs & below);
+      S.dl[s + i] = sd[p];
+      S.zk[s + i] = sz[p];
+      S.col[s + i] = S.perm[s + p];
+    } else if (gone) {
+      const int t = nd + __popc(bd & below);
+      S.dv[s + t] = sd[p];
+      S.dcol[s + t] = S.perm[s + p];
+    }
+    K += __popc(bs);
+    nd += __popc(bd);
+  }
+  if (lane == 0) S.K[mi] = K;
+}
+
+// New eigenvectors of one merge: columns of roots q(:, col(i)) u(i, j), deflated columns copied.  RT x CT threads, each
+// RM x CM outputs (RT RM and CT CM at least the merge's size).
+template <int RT, int CT, int RM, int CM>
+__device__ __forceinline__ void sub_vectors(const SubShared& S, const double (*q)[kSubLd], double (*t)[kSubLd], int s,
+                                            int n, int K, int lt) {
+  const int rt = lt / CT, ct = lt % CT;
+  double acc[RM][CM];
+#pragma unroll
+  for (int a = 0; a < RM; ++a)
+#pragma unroll
+    for (int b = 0; b < CM; ++b) acc[a][b] = 0.0;
+  // Rows and columns beyond the merge read in-bounds values (other blocks, zeros) that are not stored.
+#pragma unroll 4
+  for (int i = 0; i < K; ++i) {
+    const int c = s + S.col[s + i];
+    double x[RM], y[CM];
+#pragma unroll
+    for (int a = 0; a < RM; ++a) x[a] = q[min(s + rt + RT * a, kSubMax - 1)][c];
+#pragma unroll
+    for (int b = 0; b < CM; ++b) y[b] = S.u[s + i][min(s + ct + CT * b, kSubMax - 1)];
+#pragma unroll
+    for (int a = 0; a < RM; ++a)
+#pragma unroll
+      for (int b = 0; b < CM; ++b) acc[a][b] = fma(x[a], y[b], acc[a][b]);
+  }
+#pragma unroll
+  for (int b = 0; b < CM; ++b) {
+    const int j = ct + CT * b;
+    if (j >= n) continue;
+    const int c = s + S.out[s + j];
+#pragma unroll
+    for (int a = 0; a < RM; ++a) {
+      const int r = rt + RT * a;
+      if (r < n) t[s + r][c] = j < K ? acc[a][b] : q[s + r][s + S.dcol[s + j - K]];
+    }
+  }
+}
+
+// The subtrees at depth `depth` of the tree (at most kSubMax long), one CTA each, from the tridiagonal to their
+// eigenvalues and vectors, in shared memory: leaves of at most 8 by Jacobi (one warp each), then up to three levels of
+// merges.  At depth l of the subtree the CTA's threads split into 2^l groups of 512 / 2^l, one per merge, with eight
+// lanes per position: z and the merged order, deflation (one warp), eight lanes per secular root, recomputed z and vector,
+// then the product with the blocks' vectors in register tiles.  The steps and tests are those of the level kernels below.
+// What bounds it is latency: a few hundred dependent operations per level, in place of nine launches.  It took the place
+// of Jacobi leaves of 16 and the level kernels up to 64: the whole tridiagonal solve 203 -> 59 us at n = 37, 346 -> 193 at
+// 130, 548 -> 344 at 412 (with the branch-free divisions).  Leaves of 8 because a Jacobi round's latency does not depend
+// on the size, and 16 take twice the rounds.
+// The subtree's tears are those of its ends and of its leaves' ends.  Results go to dd / dnext and the diagonal block of
+// both eigenvector buffers (the entry state of the first level above), or, for the whole matrix (depth 0), straight to
+// d_out (unscaled) and z.
+__global__ void __launch_bounds__(kSubThreads, 1) dc_subtree_kernel(int ntot, int depth, const double* d,
+                                                                 const double* e, const double* scale_in,
+                                                                 double* dd, double* dnext, double* qa, double* qb, int ld,
+                                                                 double* d_out, double* z, int ldz, DeviceStatus* st) {
+  extern __shared__ __align__(16) unsigned char sub_smem[];
+  SubShared& S = *reinterpret_cast<SubShared*>(sub_smem);
+  __shared__ double red[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int lo = 0, hi = ntot;
+  tree_block(blockIdx.x, depth, lo, hi);
+  const int m = hi - lo;
+  if (m <= 0 || m > kSubMax) return;
+  double sc;
+  if (depth == 0) {  // the whole matrix: its scale is found here
+    double x = 0.0;
+    for (int i = tid; i < ntot; i += kSubThreads) x = fmax(x, fmax(fabs(d[i]), i < ntot - 1 ? fabs(e[i]) : 0.0));
+    sc = block_max(x, red);
+  } else {
+    sc = scale_in[0];
+  }
+  const double inv = sc > 0.0 ? 1.0 / sc : 1.0;
+  for (int t = tid; t < kSubMax * kSubLd; t += kSubThreads) {
+    (&S.q[0][0][0])[t] = 0.0;
+    (&S.q[1][0][0])[t] = 0.0;
+    (&S.u[0][0])[t] = 0.0;
+  }
+  __syncthreads();
+  const int L = tree_depth(m, kSubLeaf);
+  for (int i = tid; i < m; i += kSubThreads) {
+    S.q[0][i][i] = d[lo + i] * inv;
+    const double off = lo + i < ntot - 1 ? e[lo + i] * inv : 0.0;
+    S.e[i] = off;
+    if (i < m - 1) S.q[0][i][i + 1] = S.q[0][i + 1][i] = off;
+  }
+  __syncthreads();
+  {
+    int s = 0, t = m;
+    tree_block(warp, L, s, t);
+    const bool has = warp < (1 << L);
+    if (has && lane == 0) {  // tears at both ends (an inner end's neighbour loses the same)
+      if (lo + s > 0) S.q[0][s][s] -= fabs(s > 0 ? S.e[s - 1] : e[lo - 1] * inv);
+      if (lo + t < ntot) S.q[0][t - 1][t - 1] -= fabs(S.e[t - 1]);
+      if (t < m) S.q[0][t - 1][t] = S.q[0][t][t - 1] = 0.0;  // outside every leaf
+    }
+    __syncthreads();
+    if (has) sub_leaf(S, S.q[0], S.q[1], S.d[0], s, t - s);
+  }
+  __syncthreads();
+  int cur = 0;
+  for (int lev = L - 1; lev >= 0; --lev) {
+    const int tp = kSubThreads >> lev, mi = tid / tp, lt = tid - mi * tp;
+    int s = 0, t = m;
+    tree_block(mi, lev, s, t);
+    const int n = t - s, n1 = n / 2, pos = lt >> 3, g = lt & 7;
+    double(*q)[kSubLd] = S.q[cur];
+    const double* dc = S.d[cur];
+    const double beta = S.e[s + n1 - 1];
+    // z and the merged ascending order (ties keep the upper half first).
+    if (g == 0 && pos < n) {
+      const double rs2 = 0.70710678118654752440;
+      const double x = dc[s + pos];
+      double zv;
+      int b0, b1;
+      if (pos < n1) {
+        zv = q[s + n1 - 1][s + pos] * rs2;
+        b0 = n1; b1 = n;
+      } else {
+        zv = copysign(1.0, beta) * q[s + n1][s + pos] * rs2;
+        b0 = 0; b1 = n1;
+      }
+      const int base = b0;
+      while (b0 < b1) {  // second-half values < x, or first-half values <= x
+        const int mid = (b0 + b1) >> 1;
+        const double o = okey(dc[s + mid]);
+        if (pos < n1 ? o < okey(x) : o <= okey(x)) b0 = mid + 1;
+        else b1 = mid;
+      }
+      const int rank = (pos < n1 ? pos : pos - n1) + b0 - base;
+      S.sd[s + rank] = x;
+      S.sz[s + rank] = zv;
+      S.perm[s + rank] = pos;
+    }
+    if (lt == 0) S.rho[mi] = 2.0 * fabs(beta);
+    __syncthreads();
+    if (lt < 32) {
+      const double dmax = fmax(fmax(fabs(dc[s]), fabs(dc[s + n1 - 1])), fmax(fabs(dc[s + n1]), fabs(dc[s + n - 1])));
+      sub_deflate(S, mi, s, n, dmax);
+    }
+    __syncthreads();
+    const int K = S.K[mi], nrot = S.nrot[mi];
+    const double rho = S.rho[mi];
+    if (lt < n) {
+      double* row = q[s + lt] + s;
+      for (int r = 0; r < nrot; ++r) {
+        const int i = S.ri[s + r], j = S.rj[s + r];
+        const double c = S.rc[s + r], sn = S.rs[s + r], xi = row[i], xj = row[j];
+        row[i] = c * xi + sn * xj;
+        row[j] = -sn * xi + c * xj;
+      }
+    }
+    const double* dl = S.dl + s;
+    if (pos < K) {
+      int o;
+      double tau;
+      const bool ok = secular_root<0>(dl, S.zk + s, K, rho, pos, &o, &tau, nullptr);
+      if (g == 0) {
+        if (!ok) set_status(st, kStatusSecularNoConv, lo + s + pos + 1, lo + s);
+        S.org[s + pos] = o;
+        S.tau[s + pos] = tau;
+        S.lam[s + pos] = dl[o] + tau;
+      }
+    }
+    __syncthreads();
+    const unsigned mask = 0xffu << (tid & 24);
+    if (pos < K) {  // recomputed z (Gu-Eisenstat)
+      const double di = dl[pos];
+      double prod = 1.0;
+#pragma unroll 4
+      for (int j = g; j < K; j += 8) {
+        const double del = (di - dl[S.org[s + j]]) - S.tau[s + j];
+        prod *= (j == pos) ? -del : div_normal(del, j == pos ? 1.0 : di - dl[j]);
+      }
+      prod *= __shfl_xor_sync(mask, prod, 4);
+      prod *= __shfl_xor_sync(mask, prod, 2);
+      prod *= __shfl_xor_sync(mask, prod, 1);
+      if (g == 0) S.zh[s + pos] = copysign(sqrt(fmax(prod, 0.0)), S.zk[s + pos]);
+    }
+    // Final order: roots, then deflated values.
+    if (g == 1 && pos < n) {
+      int c;
+      double x;
+      if (pos < K) {
+        x = S.lam[s + pos];
+        c = pos;
+        for (int r = 0; r < n - K; ++r) c += okey(S.dv[s + r]) < okey(x);
+      } else {
+        const int w = pos - K;
+        x = S.dv[s + w];
+        c = 0;
+        for (int j = 0; j < K; ++j) c += okey(S.lam[s + j]) <= okey(x);
+        for (int r = 0; r < n - K; ++r)
+          c += (okey(S.dv[s + r]) < okey(x)) || (okey(S.dv[s + r]) == okey(x) && r < w);
+      }
+      S.out[s + pos] = c;
+      S.d[cur ^ 1][s + c] = x;
+    }
+    __syncthreads();
+    if (pos < K) {  // column pos of the rank-one eigenvectors
+      if (K == 1) {
+        if (g == 0) S.u[s][s] = 1.0;
+      } else {
+        const double dlo = dl[S.org[s + pos]], tau = S.tau[s + pos];
+        double ss = 0.0;
+#pragma unroll 4
+        for (int i = g; i < K; i += 8) {
+          const double x = div_normal(S.zh[s + i], (dl[i] - dlo) - tau);
+          S.u[s + i][s + pos] = x;
+          ss = fma(x, x, ss);
+        }
+        ss += __shfl_xor_sync(mask, ss, 4);
+        ss += __shfl_xor_sync(mask, ss, 2);
+        ss += __shfl_xor_sync(mask, ss, 1);
+        const double norm = 1.0 / sqrt(ss);
+        for (int i = g; i < K; i += 8) S.u[s + i][s + pos] *= norm;
+      }
+    }
+    __syncthreads();
+    double(*out)[kSubLd] = S.q[cur ^ 1];
+    if (lev == 0) sub_vectors<16, 32, 4, 2>(S, q, out, s, n, K, lt);
+    else if (lev == 1) sub_vectors<16, 16, 2, 2>(S, q, out, s, n, K, lt);
+    else sub_vectors<8, 16, 2, 1>(S, q, out, s, n, K, lt);
+    cur ^= 1;
+    __syncthreads();
+  }
+  const double(*q)[kSubLd] = S.q[cur];
+  if (depth == 0) {
+    const double up = sc > 0.0 ? sc : 1.0;
+    for (int i = tid; i < m; i += kSubThreads) d_out[i] = S.d[cur][i] * up;
+    for (int t = tid; t < m * m; t += kSubThreads) {
+      const int c = t / m, r = t - c * m;
+      z[(size_t)r + (size_t)c * ldz] = q[r][c];
+    }
+    return;
+  }
+  for (int i = tid; i < m; i += kSubThreads) dd[lo + i] = dnext[lo + i] = S.d[cur][i];
+  for (int t = tid; t < m * m; t += kSubThreads) {
+    const int c = t / m, r = t - c * m;
+    const size_t at = (size_t)(lo + r) + (size_t)(lo + c) * ld;
+    qa[at] = qb[at] = q[r][c];
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ partial top merge
@@ -913,7 +1306,6 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
                          int m_cols, int leaf) {
   if (n <= 0) return cudaSuccess;
   if (m_cols <= 0 || m_cols > n) m_cols = n;
-  if (leaf > kLeafMax) leaf = kLeafMax;
   if (work_bytes < stedc_work_bytes(n)) return cudaErrorInvalidValue;
   char* p = reinterpret_cast<char*>(work);
   char* pp = reinterpret_cast<char*>(plan);
@@ -1021,6 +1413,19 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
     if (err != cudaSuccess) return err;
   }
 
+  // With leaves, the levels at the subtree depth and below are one launch (for n <= kSubMax the whole solve is).
+  const int D = leaf > 1 ? tree_depth(n, kSubMax) : -1;
+  int l_first = 0;
+  if (D >= 0) {
+    err = allow_max_dynamic_smem(dc_subtree_kernel);
+    if (err != cudaSuccess) return err;
+  }
+  if (D == 0) {
+    dc_subtree_kernel<<<1, kSubThreads, sizeof(SubShared), s>>>(n, 0, d, e, nullptr, nullptr, nullptr, nullptr, nullptr, 0, d,
+                                                                z, ldz, st);
+    note_launches();
+    return cudaGetLastError();
+  }
   // Index arrays start at 0: an entry that a ranking on non-finite input might leave unwritten stays in range.
   err = cudaMemsetAsync(B.sperm, 0, (size_t)((char*)(B.rorg + n) - (char*)B.sperm), s);
   if (err != cudaSuccess) return err;
@@ -1030,14 +1435,10 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
     const int blocks = (int)std::min<size_t>((nn + 255) / 256, 4096);
     dc_identity_kernel<<<blocks, 256, 0, s>>>(n, n, B.Qa, B.Qb, B.dd, dnext); note_launches();
   }
-  // With leaves, the levels at the leaf depth and below are replaced by one direct solve per leaf block.
-  const int D = leaf_depth(n, leaf);
-  int l_first = 0;
-  if (D >= 0) {
-    const size_t lsmem = (size_t)2 * kLeafMax * (kLeafMax + 1) * sizeof(double);
-    err = allow_max_dynamic_smem(dc_leaf_kernel);
-    if (err != cudaSuccess) return err;
-    dc_leaf_kernel<<<1 << D, 256, lsmem, s>>>(n, D, d, B.ee, B.scale, B.dd, dnext, B.Qa, B.Qb, n); note_launches();
+  if (D > 0) {
+    dc_subtree_kernel<<<1 << D, kSubThreads, sizeof(SubShared), s>>>(n, D, d, e, B.scale, B.dd, dnext, B.Qa, B.Qb, n, nullptr,
+                                                                     nullptr, 0, st);
+    note_launches();
     l_first = std::max(0, L - D);  // levels[l] holds the merges at depth L - 1 - l
   }
   for (int l = l_first; l < L; ++l) {
