@@ -35,7 +35,8 @@
 // in registers leave it 6.  Eight warps instead of sixteen halve the shuffles and the cross-warp sums, and a column's
 // code is specialised on the column pairs still active, so that it is straight-line and its dependent chains interleave.
 // Whole stage, FP64, before -> after: n = 1788 7.19 -> 4.52 ms (4.0 -> 2.5 us per column), 1203 4.27 -> 2.70,
-// 619 1.88 -> 1.21, 412 1.19 -> 0.69; FP32 n = 1788 6.24 -> 3.85.
+// 619 1.88 -> 1.21, 412 1.19 -> 0.69; FP32 n = 1788 6.24 -> 3.85 (now, with the last 64 columns in registers and the
+// publication's addresses formed ahead: 4.28, 2.52, 1.03, 0.56; FP32 3.56).
 //
 // The ring has three thirds of H slots; step t uses slot t mod 3H.  In step t = bH + 1, after publishing, the owner
 // of a row puts the empty pattern back into its entries of third (b - 1) mod 3 and every thread executes a fence.
@@ -326,6 +327,12 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
   if (first_row >= n - 1 && cta > 0) return;  // no row in any step
   int ja = (n - 1 + 2 * NT - 1) / (2 * NT);  // column pairs per thread that reach below k
   T* xch = p.xch;                            // ((A x)_r, A(r, k-1)) pairs of this step
+  // Thread q publishes own row q (rows beyond the block's threads: a loop): where it finds the row's sums and its
+  // A(r, k-1), formed once, since the publication is on every CTA's critical path.
+  const int my_row = row_of(tid);
+  const T* my_sums = red + min(tid, R);
+  const T* my_col = tid < RR || tid >= R ? colk + min(tid, 7) : rows + (size_t)(tid - RR) * ldr;
+  const int my_step = tid < RR ? 0 : 1;
   T* const ring_end = p.xch + (size_t)3 * H * slot_ld;
   for (int k = n - 1; k >= k_end; --k) {
     if (last_row >= k) {
@@ -398,12 +405,15 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
       // ---- 3. publish ((A x)_r, A(r,k-1)) for own rows, one thread per row; neighbouring rows fill a 32-byte sector in
       //      one store.  The consumer forms y_r = scale (A x)_r + A(r, k-1) with the same fma as the owner.
       T ax_own = T(0), col_own = T(0);
-      for (int q = tid; q < nq; q += NT) {
+      if (tid < nq) {
+        ax_own = tree_sum<NW>(my_sums, R + 8);
+        col_own = my_col[my_step * (k - 1)];
+        st_pair(xch + 2 * (size_t)my_row, published(ax_own), published(col_own));
+      }
+      for (int q = tid + NT; q < nq; q += NT) {
         const T ax = tree_sum<NW>(red + q, R + 8);
-        const T ck = q < RR ? colk[q] : rows[(size_t)(q - RR) * ldr + (k - 1)];
-        st_pair(xch + 2 * (size_t)row_of(q), published(ax), published(ck));
-        if (q == tid) { ax_own = ax; col_own = ck; }
-        else red[q] = ax;  // more rows than threads
+        st_pair(xch + 2 * (size_t)row_of(q), published(ax), published(rows[(size_t)(q - RR) * ldr + (k - 1)]));
+        red[q] = ax;
       }
       // ---- 4. Householder vector (identical in every CTA: same data, same order).
       const T xn2 = tree_sum<NW>(bred, 1);
@@ -435,16 +445,13 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
         if (c < k) ld_pair(xch + 2 * c, y[i], col[i]);
       }
       // In the shadow of the loads: own rows' (v, y) and output entries, the scalars, the ring's upkeep.
-      for (int q = tid; q < nq; q += NT) {
-        const int r = row_of(q);
-        if (q != tid) {
-          ax_own = red[q];
-          col_own = rows[(size_t)(q - RR) * ldr + (k - 1)];
-        }
+      auto keep_row = [&](int q, int r, T ax, T ck) {
         const T v = r < k - 1 ? xsm[r] * scale : T(1);
-        vy[q] = Pair<T>{v, fma(scale, ax_own, col_own)};
+        vy[q] = Pair<T>{v, fma(scale, ax, ck)};
         p.aout[r + (size_t)k * p.lda] = r < k - 1 ? v : beta;
-      }
+      };
+      if (tid < nq) keep_row(tid, my_row, ax_own, col_own);
+      for (int q = tid + NT; q < nq; q += NT) keep_row(q, row_of(q), red[q], rows[(size_t)(q - RR) * ldr + (k - 1)]);
       if (cta == 0 && tid == NT - 1) { p.e[k - 1] = beta; p.tau[k - 1] = tau; }
       if (phase == 1) {  // empty the third that every CTA has finished reading (see above)
         if (!first_block) {
