@@ -1,4 +1,4 @@
-// Grouped GEMM kernel (see gemm.cuh): one CTA per 64 x 64 output tile of any problem of the group, the tile computed
+// Grouped GEMM kernel (see gemm.cuh): one CTA per 64 x 64 (32 x 32) output tile of any problem of the group, the tile computed
 // by tile::gemm_tile (FP64 DMMA, four-stage cp.async pipeline; gemm_tile.cuh).
 #include "gemm.cuh"
 
@@ -27,15 +27,16 @@ struct DescInline {
   __device__ const GemmDesc<T>& get(int i) const { return d[i]; }
 };
 
-template <typename T>
+template <typename T, int BT>
 constexpr size_t gemm_smem_bytes() {
-  return tile::smem_elems<T>() * sizeof(T);
+  return tile::smem_elems<T, BT>() * sizeof(T);
 }
 
-template <typename T, typename Src>
-// Three CTAs per SM (at most 168 registers per thread, 3 x 69.6 KB of pipeline stages): 12 warps per SM hide the DMMA
-// and shared-memory latencies that 2 CTAs (176 registers) left exposed; 1788^3 runs at 20-21 TFLOP/s instead of 17.
-__global__ void __launch_bounds__(kGemmThreads, 3) gemm_grouped_kernel(const __grid_constant__ Src src) {
+// Three CTAs per SM for 64 x 64 tiles (at most 168 registers per thread, 3 x 69.6 KB of pipeline stages): 12 warps per SM
+// hide the DMMA and shared-memory latencies that 2 CTAs (176 registers) left exposed; 1788^3 ran at 20-21 TFLOP/s instead
+// of 17.  32 x 32 tiles need a quarter of the registers and half the shared memory: six CTAs.
+template <typename T, typename Src, int BT>
+__global__ void __launch_bounds__(kGemmThreads, BT == 64 ? 3 : 6) gemm_grouped_kernel(const __grid_constant__ Src src) {
   extern __shared__ __align__(16) unsigned char gemm_smem[];
   __shared__ int s_prob;
   const int t = blockIdx.x;
@@ -52,36 +53,44 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_grouped_kernel(const __g
   const int local = t - p.tile_begin;
   if (local < 0 || local >= p.tiles_m * p.tiles_n) return;
   const int tm = local % p.tiles_m, tn = local / p.tiles_m;
-  tile::gemm_tile<T>(p, tm * kGemmBM, tn * kGemmBN, reinterpret_cast<T*>(gemm_smem));
+  tile::gemm_tile<T, BT>(p, tm * BT, tn * BT, reinterpret_cast<T*>(gemm_smem));
 }
 
 // The pipeline's shared memory exceeds the default 48 KB: opt in once per device and kernel instantiation.
-template <typename T, typename Src>
+template <typename T, typename Src, int BT>
 cudaError_t gemm_enable_smem() {
   static bool enabled[64];
   int dev = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
   if (dev >= 0 && dev < 64 && enabled[dev]) return cudaSuccess;
-  err = cudaFuncSetAttribute(gemm_grouped_kernel<T, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)gemm_smem_bytes<T>());
+  err = cudaFuncSetAttribute(gemm_grouped_kernel<T, Src, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)gemm_smem_bytes<T, BT>());
   if (err == cudaSuccess && dev >= 0 && dev < 64) enabled[dev] = true;
   return err;
+}
+
+template <typename T, typename Src, int BT>
+cudaError_t gemm_launch(const Src& src, int tiles, cudaStream_t s) {
+  const cudaError_t err = gemm_enable_smem<T, Src, BT>();
+  if (err != cudaSuccess) return err;
+  gemm_grouped_kernel<T, Src, BT><<<tiles, kGemmThreads, gemm_smem_bytes<T, BT>(), s>>>(src);
+  note_launches();
+  return cudaGetLastError();
 }
 
 }  // namespace
 
 template <typename T>
-void gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, cudaStream_t s) {
+void gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, int edge, cudaStream_t s) {
   if (nprob <= 0 || total_tiles <= 0) return;
   DescFromMemory<T> src{d_descs, nprob};
-  if (gemm_enable_smem<T, DescFromMemory<T>>() != cudaSuccess) return;
-  gemm_grouped_kernel<T, DescFromMemory<T>><<<total_tiles, kGemmThreads, gemm_smem_bytes<T>(), s>>>(src);
-  note_launches();
+  if (edge == 32) gemm_launch<T, DescFromMemory<T>, 32>(src, total_tiles, s);
+  else gemm_launch<T, DescFromMemory<T>, 64>(src, total_tiles, s);
 }
 
-template void gemm_grouped_launch<double>(const GemmDesc<double>*, int, int, cudaStream_t);
-template void gemm_grouped_launch<float>(const GemmDesc<float>*, int, int, cudaStream_t);
+template void gemm_grouped_launch<double>(const GemmDesc<double>*, int, int, int, cudaStream_t);
+template void gemm_grouped_launch<float>(const GemmDesc<float>*, int, int, int, cudaStream_t);
 
 template <typename T>
 GemmDesc<T> gemm_problem(int M, int N, int K, T alpha, const T* A, int lda, int transA, const T* B, int ldb,
@@ -105,27 +114,30 @@ cudaError_t gemm_group(DescArena& arena, const GemmDesc<T>* probs, int nprob, cu
   const bool inline_descs = nprob <= kGemmInlineMax;
   if (!inline_descs && !arena.take((size_t)nprob * sizeof(GemmDesc<T>), &h, &d)) return cudaErrorMemoryAllocation;
   GemmDesc<T>* hd = inline_descs ? inl.d : reinterpret_cast<GemmDesc<T>*>(h);
+  long tiles64 = 0, tiles32 = 0;
+  for (int i = 0; i < nprob; ++i)
+    if (probs[i].M > 0 && probs[i].N > 0) {
+      tiles64 += gemm_tiles(probs[i].M, probs[i].N, 64);
+      tiles32 += gemm_tiles(probs[i].M, probs[i].N, 32);
+    }
+  const int edge = gemm_tile_edge<T>(tiles64, tiles32);
   int tb = 0;
   for (int i = 0; i < nprob; ++i) {
     hd[i] = probs[i];
     const bool empty = probs[i].M <= 0 || probs[i].N <= 0;
-    hd[i].tiles_m = empty ? 0 : (probs[i].M + kGemmBM - 1) / kGemmBM;
-    hd[i].tiles_n = empty ? 0 : (probs[i].N + kGemmBN - 1) / kGemmBN;
+    hd[i].tiles_m = empty ? 0 : (probs[i].M + edge - 1) / edge;
+    hd[i].tiles_n = empty ? 0 : (probs[i].N + edge - 1) / edge;
     hd[i].tile_begin = tb;
     tb += hd[i].tiles_m * hd[i].tiles_n;
   }
   if (tb == 0) return cudaSuccess;
   if (inline_descs) {
     inl.n = nprob;
-    cudaError_t e = gemm_enable_smem<T, DescInline<T>>();
-    if (e != cudaSuccess) return e;
-    gemm_grouped_kernel<T, DescInline<T>><<<tb, kGemmThreads, gemm_smem_bytes<T>(), s>>>(inl);
-    note_launches();
-    return cudaGetLastError();
+    return edge == 32 ? gemm_launch<T, DescInline<T>, 32>(inl, tb, s) : gemm_launch<T, DescInline<T>, 64>(inl, tb, s);
   }
   cudaError_t err = cudaMemcpyAsync(d, h, (size_t)nprob * sizeof(GemmDesc<T>), cudaMemcpyHostToDevice, s);
   if (err != cudaSuccess) return err;
-  gemm_grouped_launch<T>(reinterpret_cast<GemmDesc<T>*>(d), nprob, tb, s);
+  gemm_grouped_launch<T>(reinterpret_cast<GemmDesc<T>*>(d), nprob, tb, edge, s);
   return cudaGetLastError();
 }
 

@@ -45,12 +45,26 @@ struct GemmDesc {
 constexpr int kGemmBM = 64, kGemmBN = 64, kGemmBK = 16, kGemmThreads = 128;
 constexpr int kGemmInlineMax = 32;  // descriptors passed by value in the launch (parameter space)
 
-inline int gemm_tiles(int m, int n) {
-  return ((m + kGemmBM - 1) / kGemmBM) * ((n + kGemmBN - 1) / kGemmBN);
+inline long gemm_tiles(int m, int n, int edge) { return (long)((m + edge - 1) / edge) * ((n + edge - 1) / edge); }
+
+// Edge of the output tiles of a launch whose problems have tiles64 tiles of 64 x 64, or tiles32 of 32 x 32, together.  The
+// cost of a K step (16) on the busiest of the 148 SMs, in units of a 32 x 32 tile (FP64 0.24 us, FP32 0.30): one, two,
+// three 64 x 64 tiles together take 4.4, 5.6, 8.5 units (FP64: 1.05, 1.32, 2.0 us; a lone CTA waits for its own loads and
+// products), or 3.5, 4.4, 6.3 (FP32); a fourth waits for a place; 32 x 32 tiles take 1 each.  So 32 x 32 wins up to about
+// 200 tiles of 64 x 64 (FP32: 100), and where a few tiles would start a second wave.  FP64: 412^3 16.5 us against 28.8,
+// 130^3 6.2 / 12.3, 840^3 57 / 70, 1350^3 222 / 269; but 940^3 85 / 78, 1788^3 465 / 425.
+template <typename T>
+int gemm_tile_edge(long tiles64, long tiles32) {
+  constexpr bool f64 = sizeof(T) == 8;
+  const double cost[3] = {f64 ? 4.4 : 3.5, f64 ? 5.6 : 4.4, f64 ? 8.5 : 6.3};
+  const long slots = 3 * 148, rest = tiles64 % slots;
+  const double c64 = (double)(tiles64 / slots) * cost[2] + (rest > 0 ? cost[(rest - 1) / 148] : 0.0);
+  return (double)((tiles32 + 147) / 148) < c64 ? 32 : 64;
 }
 
-// Launch a group: descs (device) holds nprob descriptors whose tile_begin are a prefix sum; total_tiles their sum.
+// Launch a group: descs (device) holds nprob descriptors whose tiles_m, tiles_n count tiles of `edge` and whose
+// tile_begin are their prefix sum; total_tiles their sum.
 template <typename T>
-void gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, cudaStream_t s);
+void gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, int edge, cudaStream_t s);
 
 }  // namespace xtbeig

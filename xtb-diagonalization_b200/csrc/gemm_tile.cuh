@@ -1,8 +1,14 @@
-// One 64 x 64 output tile of C = alpha op(A) op(B) + beta C computed by a whole CTA of kGemmThreads (4 warps of
-// 32 x 32).  Shared by the grouped GEMM kernel and by the persistent Cholesky kernel, which calls it from inside its
-// own phases.  FP64 issues mma.sync.m8n8k4 f64 (layout of the PTX ISA's m8n8k4 .f64 shape: A row = lane/4,
+// One BT x BT output tile (64 or 32) of C = alpha op(A) op(B) + beta C computed by a whole CTA of kGemmThreads (4 warps
+// of BT/2 x BT/2).  Shared by the grouped GEMM kernel and by the persistent Cholesky kernel, which calls it from inside
+// its own phases.  FP64 issues mma.sync.m8n8k4 f64 (layout of the PTX ISA's m8n8k4 .f64 shape: A row = lane/4,
 // col = lane%4; B row = lane%4, col = lane/4; C row = lane/4, cols 2*(lane%4) + {0,1}); FP32 uses CUDA-core FMAs on
 // the same tiling (the FP32 ABI must keep FP32 rounding).  K runs through a STAGES-deep cp.async pipeline.
+//
+// What bounds it: with one CTA per SM (small problems) the latency of a K step, with three the FP64 pipe.  A thread's
+// source pointers are formed once per tile and stepped along K, and the tests for the matrix's edge and the triangles
+// are made only in the K steps that need them: formed per element, the addresses took longer than the step's
+// multiplications (a lone CTA 1.9 us per step of 16, now 1.05; 1788^3 at 20.9 TFLOP/s, now 26.9).  Tiles of 32 x 32
+// spread a small problem over four times as many SMs (gemm_tile_edge).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -11,15 +17,17 @@
 namespace xtbeig {
 namespace tile {
 
-constexpr int BM = kGemmBM, BN = kGemmBN, BK = kGemmBK;
-constexpr int SA = BM + 4;  // smem row stride (elements): 68 = 4 (mod 16) keeps each half-warp's fragment loads
-constexpr int SB = BN + 4;  //   on 16 distinct 8-byte banks
+constexpr int BK = kGemmBK;
 // Three K-tiles in flight while one is consumed hides L2/HBM latency behind the DMMA loop.
 constexpr int STAGES = 4;
 
-template <typename T>
+// smem row stride (elements) of a K-tile: 4 (mod 16) keeps each half-warp's fragment loads on 16 distinct 8-byte banks.
+template <int BT>
+constexpr int kStride = BT + 4;
+
+template <typename T, int BT = kGemmBM>
 constexpr size_t smem_elems() {
-  return (size_t)STAGES * (BK * SA + BK * SB);
+  return (size_t)STAGES * 2 * BK * kStride<BT>;
 }
 
 __device__ __forceinline__ void cp_async_8(void* smem, const void* gmem, bool pred) {
@@ -47,38 +55,60 @@ __device__ __forceinline__ void cp_elem<float>(float* smem, const float* gmem, b
   cp_async_4(smem, gmem, pred);
 }
 
-// A masked element that is not loaded must still be zero in shared memory: cp.async with src-size 0 zero-fills.
-template <typename T>
-__device__ __forceinline__ void load_tiles(const GemmDesc<T>& p, T* As, T* Bs, int m0, int n0, int k0) {
-  const int tid = threadIdx.x;
-  const int M = p.M, N = p.N, K = p.K, mode = p.mode;
-#pragma unroll
-  for (int i = 0; i < (BM * BK) / kGemmThreads; ++i) {
-    int e = tid + i * kGemmThreads;
-    int m, k;
-    if (!p.transA) { m = e % BM; k = e / BM; } else { k = e % BK; m = e / BK; }
-    int gm = m0 + m, gk = k0 + k;
-    bool ok = gm < M && gk < K;
-    if (mode & kTriAUpper) ok = ok && gk >= gm;
-    if (mode & kTriALower) ok = ok && gk <= gm;
-    const T* src = p.A;
-    if (ok) src = p.transA ? p.A + gk + (size_t)gm * p.lda : p.A + gm + (size_t)gk * p.lda;
-    cp_elem<T>(As + k * SA + m, src, ok);
+// One operand's share of a thread: element i of a K-tile is (row r + i dr, k kk + i dk) of the operand seen as rows x K
+// (op(A)'s rows or op(B)'s columns), with the smaller index running along memory.
+template <typename T, int BT>
+struct Loader {
+  static constexpr int E = BT * BK / kGemmThreads;
+  const T* ptr;        // element 0 of K-tile 0 (k = klo)
+  size_t step;         // elements between consecutive i
+  size_t advance;      // elements per K-tile
+  int r, kk, dr, dk;   // element 0's row (within the tile) and k (within the K-tile), and their steps
+
+  // along_k: k runs along memory (transposed A, plain B).
+  __device__ __forceinline__ void init(const T* base, int ld, bool along_k, int r0, int klo) {
+    const int tid = threadIdx.x;
+    if (along_k) {
+      // Half a warp takes 4 rows x 4 k: 16 distinct banks of the transposed K-tile, whole sectors of memory.
+      kk = (tid & 3) | ((tid >> 2) & 12);
+      r = ((tid >> 2) & 3) | ((tid >> 4) & ~3);
+      dr = kGemmThreads / BK;
+      dk = 0;
+      ptr = base + (klo + kk) + (size_t)(r0 + r) * ld;
+      step = (size_t)dr * ld;
+      advance = BK;
+    } else {
+      r = tid % BT;
+      kk = tid / BT;
+      dr = 0;
+      dk = kGemmThreads / BT;
+      ptr = base + (r0 + r) + (size_t)(klo + kk) * ld;
+      step = (size_t)dk * ld;
+      advance = (size_t)BK * ld;
+    }
   }
+  // The K-tile at k0 (kt tiles after klo) into dst[k][row].  full: every element lies in the matrix and the kept
+  // triangle.  keep_ge / keep_le: only k >= row / k <= row.  An element that is not loaded is zero-filled (source size 0).
+  __device__ __forceinline__ void load(T* dst, const T* base, int kt, int k0, int r0, int R, int K, bool full,
+                                       bool keep_ge, bool keep_le) const {
+    const T* src = ptr + (size_t)kt * advance;
+    T* d = dst + kk * kStride<BT> + r;
+    const int dstep = dk * kStride<BT> + dr;
+    if (full) {
 #pragma unroll
-  for (int i = 0; i < (BN * BK) / kGemmThreads; ++i) {
-    int e = tid + i * kGemmThreads;
-    int n, k;
-    if (!p.transB) { k = e % BK; n = e / BK; } else { n = e % BN; k = e / BN; }
-    int gn = n0 + n, gk = k0 + k;
-    bool ok = gn < N && gk < K;
-    if (mode & kTriBUpper) ok = ok && gk <= gn;
-    if (mode & kTriBLower) ok = ok && gk >= gn;
-    const T* src = p.B;
-    if (ok) src = p.transB ? p.B + gn + (size_t)gk * p.ldb : p.B + gk + (size_t)gn * p.ldb;
-    cp_elem<T>(Bs + k * SB + n, src, ok);
+      for (int i = 0; i < E; ++i) cp_elem<T>(d + i * dstep, src + i * step, true);
+    } else {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int gr = r0 + r + i * dr, gk = k0 + kk + i * dk;
+        bool ok = gr < R && gk < K;
+        if (keep_ge) ok = ok && gk >= gr;
+        if (keep_le) ok = ok && gk <= gr;
+        cp_elem<T>(d + i * dstep, ok ? src + i * step : base, ok);
+      }
+    }
   }
-}
+};
 
 __device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -86,46 +116,46 @@ __device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-template <typename T>
+template <typename T, int MI, int ST>
 struct Frag;
 
-template <>
-struct Frag<double> {
-  __device__ __forceinline__ static void step(double (&acc)[4][4][2], const double* As, const double* Bs, int kk,
+template <int MI, int ST>
+struct Frag<double, MI, ST> {
+  __device__ __forceinline__ static void step(double (&acc)[MI][MI][2], const double* As, const double* Bs, int kk,
                                               int wm, int wn, int lane) {
-    double a[4], b[4];
+    double a[MI], b[MI];
     const int kr = kk * 4 + (lane & 3), g = lane >> 2;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = As[kr * SA + wm * 32 + i * 8 + g];
+    for (int i = 0; i < MI; ++i) a[i] = As[kr * ST + wm * MI * 8 + i * 8 + g];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = Bs[kr * SB + wn * 32 + j * 8 + g];
+    for (int j = 0; j < MI; ++j) b[j] = Bs[kr * ST + wn * MI * 8 + j * 8 + g];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) mma_f64(acc[i][j], a[i], b[j]);
+      for (int j = 0; j < MI; ++j) mma_f64(acc[i][j], a[i], b[j]);
   }
 };
 
-template <>
-struct Frag<float> {
-  __device__ __forceinline__ static void step(float (&acc)[4][4][2], const float* As, const float* Bs, int kk,
+template <int MI, int ST>
+struct Frag<float, MI, ST> {
+  __device__ __forceinline__ static void step(float (&acc)[MI][MI][2], const float* As, const float* Bs, int kk,
                                               int wm, int wn, int lane) {
     const int g = lane >> 2, c2 = (lane & 3) * 2;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int kr = kk * 4 + q;
-      float a[4], b0[4], b1[4];
+      float a[MI], b0[MI], b1[MI];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kr * SA + wm * 32 + i * 8 + g];
+      for (int i = 0; i < MI; ++i) a[i] = As[kr * ST + wm * MI * 8 + i * 8 + g];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        b0[j] = Bs[kr * SB + wn * 32 + j * 8 + c2];
-        b1[j] = Bs[kr * SB + wn * 32 + j * 8 + c2 + 1];
+      for (int j = 0; j < MI; ++j) {
+        b0[j] = Bs[kr * ST + wn * MI * 8 + j * 8 + c2];
+        b1[j] = Bs[kr * ST + wn * MI * 8 + j * 8 + c2 + 1];
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < MI; ++j) {
           acc[i][j][0] = fmaf(a[i], b0[j], acc[i][j][0]);
           acc[i][j][1] = fmaf(a[i], b1[j], acc[i][j][1]);
         }
@@ -133,50 +163,64 @@ struct Frag<float> {
   }
 };
 
-// The tile at (m0, n0) of problem p, by all kGemmThreads threads of the CTA.  smem holds smem_elems<T>() elements.
+// The tile at (m0, n0) of problem p, by all kGemmThreads threads of the CTA.  smem holds smem_elems<T, BT>() elements.
 // Returns after a __syncthreads, so the caller may reuse smem at once.  Tiles wholly outside C, or below the diagonal
 // under kCUpper, return without touching memory (uniformly for the CTA).
-template <typename T>
+template <typename T, int BT = kGemmBM>
 __device__ void gemm_tile(const GemmDesc<T>& p, int m0, int n0, T* smem) {
+  constexpr int MI = BT / 16, ST = kStride<BT>, KT = BK * ST;
   if (m0 >= p.M || n0 >= p.N) return;
-  if ((p.mode & kCUpper) && m0 > n0 + BN - 1) return;
-  T* As = smem;                   // [STAGES][BK * SA]
-  T* Bs = As + STAGES * BK * SA;  // [STAGES][BK * SB]
+  if ((p.mode & kCUpper) && m0 > n0 + BT - 1) return;
+  T* As = smem;                // [STAGES][BK][ST]
+  T* Bs = As + STAGES * KT;    // [STAGES][BK][ST]
+  const int mode = p.mode;
   int klo = 0, khi = p.K;
-  if (p.mode & kTriAUpper) klo = max(klo, m0);
-  if (p.mode & kTriBLower) klo = max(klo, n0);
-  if (p.mode & kTriALower) khi = min(khi, m0 + BM);
-  if (p.mode & kTriBUpper) khi = min(khi, n0 + BN);
+  if (mode & kTriAUpper) klo = max(klo, m0);
+  if (mode & kTriBLower) klo = max(klo, n0);
+  if (mode & kTriALower) khi = min(khi, m0 + BT);
+  if (mode & kTriBUpper) khi = min(khi, n0 + BT);
   klo = (klo / BK) * BK;
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = warp & 1, wn = warp >> 1;
-  T acc[4][4][2];
+  T acc[MI][MI][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = T(0);
+    for (int j = 0; j < MI; ++j) acc[i][j][0] = acc[i][j][1] = T(0);
 
   const int nk = khi > klo ? (khi - klo + BK - 1) / BK : 0;
   if (nk > 0) {
-#pragma unroll
+    Loader<T, BT> la, lb;
+    la.init(p.A, p.lda, p.transA != 0, m0, klo);
+    lb.init(p.B, p.ldb, p.transB == 0, n0, klo);
+    const bool fit_a = m0 + BT <= p.M, fit_b = n0 + BT <= p.N;
+    auto load = [&](int kt, int buf) {
+      const int k0 = klo + kt * BK;
+      const bool fit_k = k0 + BK <= p.K;
+      // A K-tile wholly on the kept side of a triangle needs no test.
+      const bool a_ge = (mode & kTriAUpper) && k0 < m0 + BT - 1, a_le = (mode & kTriALower) && k0 + BK - 1 > m0;
+      const bool b_le = (mode & kTriBUpper) && k0 + BK - 1 > n0, b_ge = (mode & kTriBLower) && k0 < n0 + BT - 1;
+      la.load(As + buf * KT, p.A, kt, k0, m0, p.M, p.K, fit_a && fit_k && !a_ge && !a_le, a_ge, a_le);
+      lb.load(Bs + buf * KT, p.B, kt, k0, n0, p.N, p.K, fit_b && fit_k && !b_ge && !b_le, b_ge, b_le);
+    };
+#pragma unroll 1
     for (int st = 0; st < STAGES - 1; ++st) {
-      if (st < nk) load_tiles<T>(p, As + st * BK * SA, Bs + st * BK * SB, m0, n0, klo + st * BK);
+      if (st < nk) load(st, st);
       cp_async_commit();
     }
+    int cur = 0;
+#pragma unroll 1
     for (int it = 0; it < nk; ++it) {
       cp_async_wait<STAGES - 2>();  // K-tile `it` has landed
       __syncthreads();              // ... for every thread, and K-tile it-1's buffer is free
       const int pf = it + STAGES - 1;
-      if (pf < nk) {
-        const int b = pf % STAGES;
-        load_tiles<T>(p, As + b * BK * SA, Bs + b * BK * SB, m0, n0, klo + pf * BK);
-      }
+      if (pf < nk) load(pf, (cur + STAGES - 1) % STAGES);
       cp_async_commit();
-      const int cur = it % STAGES;
 #pragma unroll
       for (int kk = 0; kk < BK / 4; ++kk)
-        Frag<T>::step(acc, As + cur * BK * SA, Bs + cur * BK * SB, kk, wm, wn, lane);
+        Frag<T, MI, ST>::step(acc, As + cur * KT, Bs + cur * KT, kk, wm, wn, lane);
+      cur = (cur + 1) % STAGES;
     }
     cp_async_wait<0>();
   }
@@ -184,23 +228,38 @@ __device__ void gemm_tile(const GemmDesc<T>& p, int m0, int n0, T* smem) {
 
   const T alpha = p.alpha, beta = p.beta;
   const int g = lane >> 2, c2 = (lane & 3) * 2;
+  // Every read of C before the first write: they are the same addresses, but the compiler cannot tell the elements apart.
+  if (beta != T(0)) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + wm * 32 + i * 8 + g;
-    if (gm >= p.M) continue;
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < MI; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int gm = m0 + wm * MI * 8 + i * 8 + g, gn = n0 + wn * MI * 8 + j * 8 + c2 + c;
+          const bool in = gm < p.M && gn < p.N && !((mode & kCUpper) && gm > gn);
+          const T old = in ? p.C[gm + (size_t)gn * p.ldc] : T(0);
+          acc[i][j][c] = alpha * acc[i][j][c] + beta * old;
+        }
+  } else {
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < MI; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) acc[i][j][c] *= alpha;
+  }
+#pragma unroll
+  for (int i = 0; i < MI; ++i) {
+    const int gm = m0 + wm * MI * 8 + i * 8 + g;
+#pragma unroll
+    for (int j = 0; j < MI; ++j)
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        const int gn = n0 + wn * 32 + j * 8 + c2 + c;
-        if (gn >= p.N) continue;
-        if ((p.mode & kCUpper) && gm > gn) continue;  // kCUpper updates the upper triangle only
-        T* dst = p.C + gm + (size_t)gn * p.ldc;
-        T v = alpha * acc[i][j][c];
-        if (beta != T(0)) v += beta * *dst;
-        *dst = v;
+        const int gn = n0 + wn * MI * 8 + j * 8 + c2 + c;
+        if (gm < p.M && gn < p.N && !((mode & kCUpper) && gm > gn))  // kCUpper updates the upper triangle only
+          p.C[gm + (size_t)gn * p.ldc] = acc[i][j][c];
       }
-    }
   }
 }
 

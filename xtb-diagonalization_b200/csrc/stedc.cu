@@ -1359,7 +1359,7 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
   // Stage all static per-level data in one pinned buffer, one upload.
   size_t need = 0;
   std::vector<size_t> offPos(L), offMer(L), offG(L);
-  std::vector<int> tiles(L);
+  std::vector<int> tiles(L), edges(L);
   for (int l = 0; l < L; ++l) {
     offPos[l] = need; need += (size_t)n * sizeof(int);
     offMer[l] = need; need += levels[l].merges.size() * sizeof(MergeDesc);
@@ -1376,6 +1376,12 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
       std::memcpy(h + offMer[l], ms.data(), ms.size() * sizeof(MergeDesc));
     }
     GemmDesc<double>* g = upload_plan ? reinterpret_cast<GemmDesc<double>*>(h + offG[l]) : nullptr;
+    long tiles64 = 0, tiles32 = 0;
+    for (const auto& m : ms) {
+      tiles64 += gemm_tiles(m.n1, m.n1 + m.n2, 64) + gemm_tiles(m.n2, m.n1 + m.n2, 64);
+      tiles32 += gemm_tiles(m.n1, m.n1 + m.n2, 32) + gemm_tiles(m.n2, m.n1 + m.n2, 32);
+    }
+    const int edge = edges[l] = gemm_tile_edge<double>(tiles64, tiles32);
     int tb = 0;
     for (size_t mi = 0; mi < ms.size(); ++mi) {
       if (pos)
@@ -1383,7 +1389,7 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
       const int nmax = ms[mi].n1 + ms[mi].n2;
       for (int half = 0; half < 2; ++half) {
         const int mrows = half == 0 ? ms[mi].n1 : ms[mi].n2;
-        const int tm = (mrows + kGemmBM - 1) / kGemmBM, tn = (nmax + kGemmBN - 1) / kGemmBN;
+        const int tm = (mrows + edge - 1) / edge, tn = (nmax + edge - 1) / edge;
         if (g) {
           GemmDesc<double>& gd = g[2 * mi + half];
           std::memset(&gd, 0, sizeof(gd));
@@ -1465,7 +1471,7 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
     if (partial) {
       dc_partial_kernel<<<1, 1024, 0, s>>>(B, m_cols); note_launches();
     }
-    gemm_grouped_launch<double>(B.gdesc, 2 * nm, tiles[l], s);
+    gemm_grouped_launch<double>(B.gdesc, 2 * nm, tiles[l], edges[l], s);
     dc_order_kernel<<<dim3(nm, (maxn + 255) / 256), 256, 0, s>>>(B, dnext); note_launches();
     dc_copy_kernel<<<dim3(nm, std::min(partial ? m_cols : maxn, 65535)), 256, 0, s>>>(B, partial ? m_cols : n);
     note_launches();
