@@ -263,7 +263,20 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const __grid_con
   }
   __syncwarp();
 
-  // Epilogue: every warp drains its 32 accumulator rows.
+  // Epilogue: every warp drains its 32 accumulator rows, 32 columns at a time.  With beta, a chunk's old values of C are
+  // loaded together, one chunk ahead of their use (the first while the last MMAs run): read and written element by
+  // element, each load waited for the store before it and a launch took 53 us longer (one tile: 66 us instead of 13.6).
+  const int row = m0 + warp * 32 + lane;
+  const float alpha = pr.alpha, beta = pr.beta;
+  float old[32];
+  auto load_c = [&](int c) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const int col = n0 + c + j;
+      old[j] = row < pr.M && col < pr.N ? pr.C[row + (size_t)col * pr.ldc] : 0.f;
+    }
+  };
+  if (beta != 0.f) load_c(0);
   bool have = nk > 0;
   if (have) {
     // Warp-uniform outcome: the TMEM loads below are .sync.aligned, so either every lane reads or none does.
@@ -272,8 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const __grid_con
     umma::tc_fence_after();
   }
   __syncwarp();
-  const int row = m0 + warp * 32 + lane;
-  const float alpha = pr.alpha, beta = pr.beta;
+#pragma unroll 1
   for (int c = 0; c < kBN; c += 32) {
     uint32_t r[32];
     if (have) {
@@ -282,16 +294,19 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const __grid_con
 #pragma unroll
       for (int j = 0; j < 32; ++j) r[j] = 0u;
     }
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = alpha * __uint_as_float(r[j]);
+    if (beta != 0.f) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = fmaf(beta, old[j], v[j]);
+      if (c + 32 < kBN) load_c(c + 32);
+    }
     if (row < pr.M) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int col = n0 + c + j;
-        if (col < pr.N) {
-          float* cp = pr.C + row + (size_t)col * pr.ldc;
-          float v = alpha * __uint_as_float(r[j]);
-          if (beta != 0.f) v = fmaf(beta, *cp, v);
-          *cp = v;
-        }
+        if (col < pr.N) pr.C[row + (size_t)col * pr.ldc] = v[j];
       }
     }
   }
