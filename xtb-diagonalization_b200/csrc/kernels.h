@@ -189,6 +189,9 @@ struct OrmtrWork {
 };
 template <typename T>
 size_t ormtr_work_elems(int n, int m, int nb);
+// Shared memory of the kernel that forms a block's factor (wy.cuh): nb x nb entries in columns of nb + kWyPad, and nb.
+constexpr int kWyPad = 4;
+inline size_t wy_factor_smem(int nb, size_t elem) { return ((size_t)nb * (nb + kWyPad) + nb) * elem; }
 template <typename T>
 OrmtrWork<T> ormtr_carve(T* base, int n, int m, int nb);
 template <typename T>

@@ -90,10 +90,9 @@ cudaError_t ormtr_prepare(int n, const T* a, int lda, const T* tau, int nb, Ormt
   cudaError_t err = gemm_run(arena, tc, probs.data(), (int)probs.size(), s);
   if (err != cudaSuccess) return err;
   {
-    const size_t smem = ((size_t)nb * (nb + 1) + nb) * sizeof(T);
     err = allow_max_dynamic_smem(wy_factor_kernel<T>);
     if (err != cudaSuccess) return err;
-    wy_factor_kernel<T><<<nblocks, 256, smem, s>>>(nm1, nb, tau, w.Y, S, w.Tf); note_launches();
+    wy_factor_kernel<T><<<nblocks, kWyThreads, wy_factor_smem(nb, sizeof(T)), s>>>(nm1, nb, tau, w.Y, S, w.Tf); note_launches();
   }
   // Y_b = V_b T_b^T (op(B) = T_b^T is lower triangular).
   probs.clear();
