@@ -354,11 +354,13 @@ void stage_sytrd(Call& k, int n, const T* dfull, int ldf, T* dout, int lda, T* d
   const size_t smem_cap = k.c->max_smem > 2048 ? k.c->max_smem - 2048 : k.c->max_smem;
   int grid = t_plan.sytrd_grid;
   if (grid == 0 && t_plan.batch_grid == 1) {
-    // Inside a batch the reductions of several problems share the GPU: each takes the fewest CTAs that still hold
-    // its rows in shared memory (with a margin), which also makes its grid barrier cheaper, and leaves the other SMs
-    // to the problems beside it.
-    const size_t bytes = (size_t)n * n * sizeof(T), per_cta = smem_cap * 4 / 5;
-    grid = (int)std::min<size_t>((size_t)k.c->num_sms, std::max<size_t>(4, (bytes + per_cta - 1) / per_cta));
+    // Inside a batch the reductions of several problems share the GPU: each takes the fewest CTAs (from 16 on) that still
+    // hold its rows in shared memory and registers (n = 1788: 82), and leaves the other SMs to the problems beside it.  A
+    // step's exchange costs more than its arithmetic, so a problem loses little: 24 uneven problems (n = 124 to 1788) took
+    // 59 ms with grids a fifth above what shared memory alone would hold (n = 1788: 143), 45 ms with these, 47 with a
+    // tenth more CTAs, 51 with a quarter more.
+    grid = std::min(k.c->num_sms, 16);
+    while (grid < k.c->num_sms && !sytrd_plan<T>(n, k.c->num_sms, smem_cap, grid).rows_in_smem) ++grid;
   }
   SytrdPlan pl = sytrd_plan<T>(n, k.c->num_sms, smem_cap, grid);
   if (!pl.supported) {
