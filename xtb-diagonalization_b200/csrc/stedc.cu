@@ -130,33 +130,50 @@ __global__ void dc_identity_kernel(int n, int ld, double* q, double* qb, const d
   }
 }
 
-// Block-wide exclusive scan of one int per thread; returns the exclusive prefix, *total receives the sum.
-__device__ int block_exscan(int v, int* scratch, int* total) {
+// ------------------------------------------------------------------------------------------------ deflate
+
+// Block-wide exclusive scan of four 32-bit counters per thread, two to a word; *total receives the sums.
+struct Counts {
+  unsigned long long a, b;
+};
+__device__ Counts block_exscan4(Counts v, Counts* scratch, Counts* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int x = v;
+  auto warp_scan = [&](Counts x) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long ya = __shfl_up_sync(0xffffffffu, x.a, o), yb = __shfl_up_sync(0xffffffffu, x.b, o);
+      if (lane >= o) {
+        x.a += ya;
+        x.b += yb;
+      }
+    }
+    return x;
+  };
+  const Counts x = warp_scan(v);
   __syncthreads();
   if (lane == 31) scratch[warp] = x;
   __syncthreads();
-  int wpre = 0, tot = 0;
-  for (int w = 0; w < nw; ++w) {
-    if (w < warp) wpre += scratch[w];
-    tot += scratch[w];
-  }
-  *total = tot;
-  return wpre + x - v;
+  const Counts w = warp_scan(lane < nw ? scratch[lane] : Counts{0, 0});
+  total->a = __shfl_sync(0xffffffffu, w.a, 31);
+  total->b = __shfl_sync(0xffffffffu, w.b, 31);
+  const unsigned long long pa = __shfl_sync(0xffffffffu, w.a, max(warp - 1, 0));
+  const unsigned long long pb = __shfl_sync(0xffffffffu, w.b, max(warp - 1, 0));
+  return Counts{(warp > 0 ? pa : 0) + x.a - v.a, (warp > 0 ? pb : 0) + x.b - v.b};
 }
 
-// ------------------------------------------------------------------------------------------------ deflate
+// What bounds it: one CTA's chain of dependent steps (searches, scans, the chain of close pairs), so every array that a
+// later step reads again lives in shared memory (kSmem; 32 bytes per position, merges of up to kDeflateSmemMax) and a
+// thread owns consecutive positions, which takes one scan for each list however long it is.  With the arrays in global
+// memory and five scans per 1024 positions a level took 19 us on average (n = 1788, five levels), now 11.  Larger merges
+// keep the arrays in global memory.
+constexpr int kDeflateSmemMax = 6400;
 
+template <bool kSmem>
 __global__ void __launch_bounds__(1024) dc_deflate_kernel(DcBufs B, int nmerge) {
+  extern __shared__ __align__(16) unsigned char deflate_smem[];
   __shared__ double s_red[32];
-  __shared__ int s_scan[32];
-  __shared__ int s_cnt[8];
+  __shared__ Counts s_scan[32];
+  __shared__ int s_nrot;
   const int mi = blockIdx.x;
   if (mi >= nmerge) return;
   DC_RETURN_IF_FAILED(B)
@@ -167,12 +184,27 @@ __global__ void __launch_bounds__(1024) dc_deflate_kernel(DcBufs B, int nmerge) 
   const double rho = 2.0 * fabs(beta);
   const double sgn = beta >= 0.0 ? 1.0 : -1.0;
   const double rs2 = 0.70710678118654752440;
-  const double* dd = B.dd + s;
-  double* sd = B.sd + s;
-  double* sz = B.sz + s;
-  int* sperm = B.sperm + s;
-  int* typ = B.typ + s;
+  // Sorted values and z, their columns and types; the values before the sort make room for the lists of candidates.
+  double* sd = kSmem ? reinterpret_cast<double*>(deflate_smem) : B.sd + s;
+  double* sz = kSmem ? sd + n : B.sz + s;
+  const double* dd = kSmem ? sz + n : B.dd + s;
+  int* ndl = kSmem ? reinterpret_cast<int*>(sz + n) : B.ndl + s;
+  int* clist = kSmem ? ndl + n : B.slotOf + s;  // slotOf's range of this merge is written only further down
+  int* sperm = kSmem ? clist + n : B.sperm + s;
+  int* typ = kSmem ? sperm + n : B.typ + s;
+  const int q = (n + blockDim.x - 1) / blockDim.x;  // positions per thread
+  const int p0 = min((int)threadIdx.x * q, n), p1 = min(p0 + q, n);
+  Counts tot;
 
+  if (kSmem) {
+    // Every entry starts in range: a ranking on non-finite input might leave one unwritten.
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      sz[n + i] = B.dd[s + i];
+      sd[i] = sz[i] = 0.0;
+      sperm[i] = typ[i] = 0;
+    }
+    __syncthreads();
+  }
   // z and the merge of the two ascending lists (stable: ties keep the upper half first).
   double dmax = 0.0, zmax = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -205,39 +237,41 @@ __global__ void __launch_bounds__(1024) dc_deflate_kernel(DcBufs B, int nmerge) 
   __syncthreads();
 
   // Small-z deflation, then the compacted list of candidates for pair deflation.
-  int* ndl = B.ndl + s;
   int m = 0;
-  for (int base = 0; base < n; base += blockDim.x) {
-    const int p = base + threadIdx.x;
-    int keep = 0;
-    if (p < n) {
-      keep = rho * fabs(sz[p]) > tol;
-      if (!keep) typ[p] = 4;
+  {
+    unsigned cnt = 0;
+    for (int p = p0; p < p1; ++p) {
+      if (rho * fabs(sz[p]) > tol) ++cnt;
+      else typ[p] = 4;
     }
-    int tot;
-    int pre = block_exscan(keep, s_scan, &tot);
-    if (keep) ndl[m + pre] = p;
-    m += tot;
+    int at = (int)block_exscan4(Counts{cnt, 0}, s_scan, &tot).a;
+    m = (int)tot.a;
+    for (int p = p0; p < p1; ++p)
+      if (typ[p] != 4) ndl[at++] = p;
     __syncthreads();
   }
-  // The pairs that pass the close-pair test before any rotation, compacted in pair order (the list borrows this
-  // merge's range of slotOf, which is written only further down).
-  int* clist = B.slotOf + s;
+  // The pairs that pass the close-pair test before any rotation, compacted in pair order.
   int nc = 0;
-  for (int base = 0; base < m - 1; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    int flag = 0;
-    if (i < m - 1) {
+  {
+    auto close = [&](int i) {
       const int a = ndl[i], b = ndl[i + 1];
       const double za = sz[a], zb = sz[b];
       const double t = hypot(za, zb);
       const double c = zb / t, sn = -za / t;
-      flag = fabs((sd[b] - sd[a]) * c * sn) <= tol;
-    }
-    int tot;
-    const int pre = block_exscan(flag, s_scan, &tot);
-    if (flag) clist[nc + pre] = i;
-    nc += tot;
+      return fabs((sd[b] - sd[a]) * c * sn) <= tol;
+    };
+    unsigned cnt = 0;
+    unsigned long long flags = 0;  // of the first 64 of the thread's pairs; later ones are tested again
+    for (int i = p0; i < p1 && i < m - 1; ++i)
+      if (close(i)) {
+        ++cnt;
+        if (i - p0 < 64) flags |= 1ull << (i - p0);
+      }
+    int at = (int)block_exscan4(Counts{cnt, 0}, s_scan, &tot).a;
+    nc = (int)tot.a;
+    if (cnt > 0)
+      for (int i = p0; i < p1 && i < m - 1; ++i)
+        if (i - p0 < 64 ? (flags >> (i - p0)) & 1 : close(i)) clist[at++] = i;
     __syncthreads();
   }
 
@@ -246,8 +280,8 @@ __global__ void __launch_bounds__(1024) dc_deflate_kernel(DcBufs B, int nmerge) 
   // deflate, which is the order and the set of tests of a scan over every pair.
   if (threadIdx.x == 0) {
     int nrot = 0, next = 0;
-    for (int q = 0; q < nc; ++q) {
-      int i = clist[q];
+    for (int w = 0; w < nc; ++w) {
+      int i = clist[w];
       if (i < next) continue;
       for (; i < m - 1; ++i) {
         const int a = ndl[i], b = ndl[i + 1];
@@ -270,61 +304,42 @@ __global__ void __launch_bounds__(1024) dc_deflate_kernel(DcBufs B, int nmerge) 
       }
       next = i + 1;
     }
-    s_cnt[0] = nrot;
+    s_nrot = nrot;
   }
   __syncthreads();
 
-  // Survivors in position order (their values ascend), their type-grouped GEMM slots, deflated list.
-  // Pass 1: counts per type.
-  int cnt[4] = {0, 0, 0, 0};
-  for (int p = threadIdx.x; p < n; p += blockDim.x) cnt[min(max(typ[p], 1), 4) - 1]++;
-  for (int t = 0; t < 4; ++t) {
-    int tot;
-    (void)block_exscan(cnt[t], s_scan, &tot);
-    if (threadIdx.x == 0) s_cnt[1 + t] = tot;
-    __syncthreads();
+  // Survivors in position order (their values ascend), their type-grouped GEMM slots, deflated list: one scan of the
+  // four types' counts.
+  unsigned cnt[4] = {0, 0, 0, 0};
+  for (int p = p0; p < p1; ++p) {
+    const int ty = min(max(typ[p], 1), 4);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) cnt[t] += ty == t + 1;
   }
-  const int c1 = s_cnt[1], c2 = s_cnt[2], c3 = s_cnt[3], nd = s_cnt[4];
+  const Counts pre = block_exscan4(Counts{cnt[0] | (unsigned long long)cnt[1] << 32, cnt[2] | (unsigned long long)cnt[3] << 32},
+                                   s_scan, &tot);
+  const int c1 = (int)(unsigned)tot.a, c2 = (int)(tot.a >> 32), c3 = (int)(unsigned)tot.b, nd = (int)(tot.b >> 32);
   const int K = c1 + c2 + c3;
-  // Pass 2: ordered ranks (survivor index i, per-type rank, deflated rank).
-  int run_i = 0, run_t[3] = {0, 0, 0}, run_d = 0;
-  for (int base = 0; base < n; base += blockDim.x) {
-    const int p = base + threadIdx.x;
-    const int ty = p < n ? typ[p] : 0;
-    const int isS = (ty >= 1 && ty <= 3), isD = (ty == 4);
-    int tot_s, tot_d, tot_t[3];
-    const int pre_s = block_exscan(isS, s_scan, &tot_s);
-    __syncthreads();
-    const int pre_d = block_exscan(isD, s_scan, &tot_d);
-    int pre_t[3];
-    for (int t = 0; t < 3; ++t) {
-      __syncthreads();
-      pre_t[t] = block_exscan(ty == t + 1, s_scan, &tot_t[t]);
+  int at1 = (int)(unsigned)pre.a, at2 = (int)(pre.a >> 32), at3 = (int)(unsigned)pre.b, atd = (int)(pre.b >> 32);
+  for (int p = p0; p < p1; ++p) {
+    const int ty = min(max(typ[p], 1), 4);
+    if (ty == 4) {
+      B.dval[s + atd] = sd[p];
+      B.srcCol[s + K + atd] = sperm[p];
+      ++atd;
+      continue;
     }
-    if (isS) {
-      const int i = run_i + pre_s;
-      int slot;
-      if (ty == 1) slot = run_t[0] + pre_t[0];
-      else if (ty == 2) slot = c1 + run_t[1] + pre_t[1];
-      else slot = c1 + c2 + run_t[2] + pre_t[2];
-      B.dlam[s + i] = sd[p];
-      B.zk[s + i] = sz[p];
-      B.slotOf[s + i] = slot;
-      B.srcCol[s + slot] = sperm[p];
-    } else if (isD) {
-      const int t = run_d + pre_d;
-      B.dval[s + t] = sd[p];
-      B.srcCol[s + K + t] = sperm[p];
-    }
-    run_i += tot_s;
-    run_d += tot_d;
-    for (int t = 0; t < 3; ++t) run_t[t] += tot_t[t];
-    __syncthreads();
+    const int i = at1 + at2 + at3;
+    const int slot = ty == 1 ? at1++ : ty == 2 ? c1 + at2++ : c1 + c2 + at3++;
+    B.dlam[s + i] = sd[p];
+    B.zk[s + i] = sz[p];
+    B.slotOf[s + i] = slot;
+    B.srcCol[s + slot] = sperm[p];
   }
 
   if (threadIdx.x == 0) {
     MergeInfo inf;
-    inf.K = K; inf.c1 = c1; inf.c2 = c2; inf.c3 = c3; inf.nrot = s_cnt[0]; inf.ndefl = nd; inf.rho = rho;
+    inf.K = K; inf.c1 = c1; inf.c2 = c2; inf.c3 = c3; inf.nrot = s_nrot; inf.ndefl = nd; inf.rho = rho;
     B.info[mi] = inf;
     // Merge GEMMs: Qnew(upper rows) = Qc(upper, slots [0, c1+c2)) Up(slots [0, c1+c2), 0:K);
     //              Qnew(lower rows) = Qc(lower, slots [c1, K))     Up(slots [c1, K), 0:K).   Qnew overwrites Qa.
@@ -1419,6 +1434,8 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
     if (err != cudaSuccess) return err;
   }
 
+  err = allow_max_dynamic_smem(dc_deflate_kernel<true>);
+  if (err != cudaSuccess) return err;
   // With leaves, the levels at the subtree depth and below are one launch (for n <= kSubMax the whole solve is).
   const int D = leaf > 1 ? tree_depth(n, kSubMax) : -1;
   int l_first = 0;
@@ -1455,7 +1472,12 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
     B.merges = mergesAll + (size_t)l * (n / 2 + 2);
     B.gdesc = gAll + (size_t)l * (n + 4);
     const int dthreads = maxn > 512 ? 1024 : (maxn > 128 ? 512 : 128);
-    dc_deflate_kernel<<<nm, dthreads, 0, s>>>(B, nm); note_launches();
+    if (maxn <= kDeflateSmemMax) {
+      dc_deflate_kernel<true><<<nm, dthreads, (size_t)32 * maxn, s>>>(B, nm);
+    } else {
+      dc_deflate_kernel<false><<<nm, dthreads, 0, s>>>(B, nm);
+    }
+    note_launches();
     dc_rotate_kernel<<<dim3(nm, (maxn + 127) / 128), 128, 0, s>>>(B); note_launches();
     dc_gather_kernel<<<dim3(nm, (maxn + 127) / 128, (maxn + 31) / 32), 128, 0, s>>>(B); note_launches();
     const int warps_per_block = 8;
