@@ -69,7 +69,6 @@ struct DcBufs {
   int* cand;      // pair candidate flags
   int* slotOf;    // survivor index -> GEMM slot
   int* srcCol;    // Qc column -> local source column in Qa
-  int* outSrc;    // output position -> source (j < K: root j; K + t: deflated t)
   int* rotI;
   int* rotJ;
   int* rorg;      // root j's origin pole (see rtau)
@@ -1207,51 +1206,53 @@ __global__ void __launch_bounds__(1024) dc_partial_kernel(DcBufs B, int m_cols) 
 
 // ------------------------------------------------------------------------------------------------ final order
 
-// grid (merges, column groups): rank of every root and deflated value in the merged ascending order; the CTAs of a
-// merge (blockIdx.y) split its roots and deflated values between them with a grid-stride loop.
-__global__ void dc_order_kernel(DcBufs B, double* dnext) {
+// grid (merges, columns): a CTA takes a column of the merge (root or deflated value), counts how many values lie before it
+// in the merged ascending order, and copies the column to that place of the next level's eigenvectors; columns placed from
+// col_limit on are not wanted (partial top merge).  The column is loaded while the count runs.  Bound by the copy's
+// latency; with the ranks in a kernel of their own the two took 18 us a level on average at n = 1788 (9 at n = 412), now
+// 10 (5).
+__global__ void __launch_bounds__(256) dc_place_kernel(DcBufs B, double* dnext, int col_limit) {
   DC_RETURN_IF_FAILED(B)
+  __shared__ int s_cnt[8];
+  constexpr int U = 8;
   const int mi = blockIdx.x;
   const MergeDesc md = B.merges[mi];
   const MergeInfo inf = B.info[mi];
   const int s = md.s, n = md.n1 + md.n2, K = inf.K, nd = n - K;
   const double* lam = B.lam + s;
   const double* dv = B.dval + s;
-  const int first = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;
-  for (int j = first; j < K; j += stride) {
-    const double x = lam[j];
-    int c = 0;
-    for (int t = 0; t < nd; ++t) c += okey(dv[t]) < okey(x);
-    const int rank = j + c;
-    B.outSrc[s + rank] = j;
-    dnext[s + rank] = x;
-  }
-  for (int t = first; t < nd; t += stride) {
-    const double x = dv[t];
-    int lo = 0, hi = K;  // roots <= x
-    while (lo < hi) { int m = (lo + hi) >> 1; if (okey(lam[m]) <= okey(x)) lo = m + 1; else hi = m; }
-    int c = lo;
-    for (int u = 0; u < nd; ++u) c += (okey(dv[u]) < okey(x)) || (okey(dv[u]) == okey(x) && u < t);
-    B.outSrc[s + c] = K + t;
-    dnext[s + c] = x;
-  }
-}
-
-// grid (merges, columns): copy each output column into the next level's eigenvector matrix, one column per CTA with a
-// grid-stride loop over the merge's columns; columns from col_limit on are not wanted (partial top merge).
-__global__ void dc_copy_kernel(DcBufs B, int col_limit) {
-  DC_RETURN_IF_FAILED(B)
-  const int mi = blockIdx.x;
-  const MergeDesc md = B.merges[mi];
-  const MergeInfo inf = B.info[mi];
-  const int s = md.s, n = md.n1 + md.n2, ncols = min(n, col_limit), K = inf.K;
   const size_t ld = B.ld;
-  // One column per CTA (while the grid allows): enough CTAs in flight to cover the copy's memory latency.
-  for (int c = blockIdx.y; c < ncols; c += gridDim.y) {
-    const int src = B.outSrc[s + c];
-    const double* from = (src < K ? B.Qa : B.Qc) + (size_t)s + (size_t)(s + src) * ld;
-    double* to = B.Qb + (size_t)s + (size_t)(s + c) * ld;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) to[r] = from[r];
+  for (int c = blockIdx.y; c < n; c += gridDim.y) {
+    const bool root = c < K;
+    const double* __restrict__ from = (root ? B.Qa : B.Qc) + (size_t)s + (size_t)(s + c) * ld;
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = threadIdx.x + 256 * u;
+      v[u] = r < n ? from[r] : 0.0;
+    }
+    const double x = root ? lam[c] : dv[c - K];
+    const auto kx = okey(x);
+    int cnt = 0;
+    if (root) {  // its index among the ascending roots, and the deflated values below it
+      for (int t = threadIdx.x; t < nd; t += 256) cnt += okey(dv[t]) < kx;
+    } else {     // roots up to it, deflated values below it (ties in index order)
+      for (int j = threadIdx.x; j < K; j += 256) cnt += okey(lam[j]) <= kx;
+      for (int t = threadIdx.x; t < nd; t += 256) {
+        const auto kt = okey(dv[t]);
+        cnt += kt < kx || (kt == kx && t < c - K);
+      }
+    }
+    const int rank = (root ? c : 0) + block_sum(cnt, s_cnt);
+    if (threadIdx.x == 0) dnext[s + rank] = x;
+    if (rank >= col_limit) continue;
+    double* __restrict__ to = B.Qb + (size_t)s + (size_t)(s + rank) * ld;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = threadIdx.x + 256 * u;
+      if (r < n) to[r] = v[u];
+    }
+    for (int r = threadIdx.x + 256 * U; r < n; r += 256) to[r] = from[r];
   }
 }
 
@@ -1298,7 +1299,7 @@ size_t stedc_work_bytes(int n) {
   for (int i = 0; i < 4; ++i) add(nn * sizeof(double));  // Qa Qb Qc Up
   for (int i = 0; i < 11; ++i) add(n * sizeof(double));  // rtau sd sz dlam zk zh lam dval rotc rots dnext
   add(sizeof(double) * 4);             // scale
-  for (int i = 0; i < 10; ++i) add(n * sizeof(int));     // sperm typ ndl cand slotOf srcCol outSrc rotI rotJ rorg
+  for (int i = 0; i < 9; ++i) add(n * sizeof(int));     // sperm typ ndl cand slotOf srcCol rotI rotJ rorg
   // per level: posMerge, merges, info, gemm descriptors (levels <= 32)
   add((size_t)32 * n * sizeof(int));
   add((size_t)32 * (n / 2 + 2) * sizeof(MergeDesc));
@@ -1352,7 +1353,6 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
   B.cand = carve<int>(p, n);
   B.slotOf = carve<int>(p, n);
   B.srcCol = carve<int>(p, n);
-  B.outSrc = carve<int>(p, n);
   B.rotI = carve<int>(p, n);
   B.rotJ = carve<int>(p, n);
   B.rorg = carve<int>(p, n);
@@ -1494,8 +1494,7 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
       dc_partial_kernel<<<1, 1024, 0, s>>>(B, m_cols); note_launches();
     }
     gemm_grouped_launch<double>(B.gdesc, 2 * nm, tiles[l], edges[l], s);
-    dc_order_kernel<<<dim3(nm, (maxn + 255) / 256), 256, 0, s>>>(B, dnext); note_launches();
-    dc_copy_kernel<<<dim3(nm, std::min(partial ? m_cols : maxn, 65535)), 256, 0, s>>>(B, partial ? m_cols : n);
+    dc_place_kernel<<<dim3(nm, std::min(maxn, 65535)), 256, 0, s>>>(B, dnext, partial ? m_cols : n);
     note_launches();
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
