@@ -43,7 +43,11 @@ constexpr int kBM = 128, kBN = 128, kBK = 32, kStages = 3, kThreads = 128;
 constexpr int kTileBytes = kBM * kBK * 4;          // one operand tile (A or B, hi or lo): 16 KB
 constexpr int kStageBytes = 4 * kTileBytes;        // A hi, A lo, B hi, B lo
 constexpr int kSmemBytes = kStages * kStageBytes + 1024;
-constexpr int kMaxProbs = 8;
+// Problems per launch.  The descriptors travel as kernel parameters (576 bytes per problem, 32 KB at most), so few problems
+// take the small form and the Gram matrices of a whole back-transformation (86 at n = 1788) two launches of the large
+// one instead of eleven (mixed solve at n = 1788: 8402 -> 8300 us; the stream that
+// forms X Q beside the divide and conquer ends 200 us earlier).
+constexpr int kFewProbs = 8, kManyProbs = 48;
 constexpr uint32_t kTmemCols = 128;
 
 struct alignas(64) UProb {
@@ -58,8 +62,9 @@ struct alignas(64) UProb {
   int tiles_m, tiles_n, tile_begin;
 };
 
+template <int kMax>
 struct UParams {
-  UProb p[kMaxProbs];
+  UProb p[kMax];
   int nprob;
   int passes;
   DeviceStatus* st;
@@ -74,13 +79,15 @@ struct SplitJob {
   int keep;  // 0 all, 1 upper (r <= c), 2 lower (r >= c)
 };
 
+template <int kMax>
 struct SplitParams {
-  SplitJob j[2 * kMaxProbs];
+  SplitJob j[2 * kMax];
   int njobs;
   int passes;
 };
 
-__global__ void umma_split_kernel(const __grid_constant__ SplitParams P) {
+template <int kMax>
+__global__ void umma_split_kernel(const __grid_constant__ SplitParams<kMax> P) {
   const SplitJob& J = P.j[blockIdx.y];
   const size_t total = (size_t)J.ldp * J.cols;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -104,13 +111,15 @@ struct SplitJob16 {
   int keep;      // 0 all, 1 k >= mn, 2 k <= mn
 };
 
+template <int kMax>
 struct Split16Params {
-  SplitJob16 j[2 * kMaxProbs];
+  SplitJob16 j[2 * kMax];
   int njobs;
   int pieces;
 };
 
-__global__ void umma_split_bf16_kernel(const __grid_constant__ Split16Params P) {
+template <int kMax>
+__global__ void umma_split_bf16_kernel(const __grid_constant__ Split16Params<kMax> P) {
   const SplitJob16& J = P.j[blockIdx.y];
   const size_t total = (size_t)J.ldk * J.MN;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -125,12 +134,13 @@ __global__ void umma_split_bf16_kernel(const __grid_constant__ Split16Params P) 
   }
 }
 
-__device__ __forceinline__ void record_timeout(const UParams& P, int where) {
+template <int kMax>
+__device__ __forceinline__ void record_timeout(const UParams<kMax>& P, int where) {
   set_status(P.st, kStatusBarrierTimeout, 0, where);
 }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const __grid_constant__ UParams P) {
+template <bool kBf16, int kMax>
+__global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const __grid_constant__ UParams<kMax> P) {
   constexpr int kBKe = kBf16 ? 64 : kBK;  // K elements per stage (128 bytes per tile row either way)
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kStages];
@@ -398,7 +408,6 @@ OperandShape shape_b(const GemmDesc<float>& p) {
 
 size_t operand_elems(const OperandShape& s) { return 2 * up64((size_t)pad4(s.rows) * std::max(s.cols, 1)); }
 
-bool g_smem_set[2][64];
 
 }  // namespace
 
@@ -411,128 +420,144 @@ size_t umma_work_elems(const GemmDesc<float>* probs, int nprob) {
   return e;
 }
 
+namespace {
+
+// One launch: cnt <= kMax problems whose operands fit in work.
+template <int kMax>
+cudaError_t umma_launch(const GemmDesc<float>* probs, int cnt, int passes, bool bf16, float* work, DeviceStatus* st,
+                        uint64_t limit_ns, cudaStream_t s) {
+  static bool smem_set[2][64];
+  UParams<kMax> up;
+  memset(&up, 0, sizeof(up));
+  SplitParams<kMax> sp;
+  memset(&sp, 0, sizeof(sp));
+  sp.passes = passes;
+  Split16Params<kMax> sp16;
+  memset(&sp16, 0, sizeof(sp16));
+  sp16.pieces = passes == 3 ? 2 : 1;
+  float* w = work;
+  int tb = 0, used = 0, max_total = 0;
+  for (int i = 0; i < cnt; ++i) {
+    const GemmDesc<float>& p = probs[i];
+    if (p.M <= 0 || p.N <= 0) continue;
+    UProb& q = up.p[used];
+    q.C = p.C;
+    q.ldc = p.ldc;
+    q.M = p.M;
+    q.N = p.N;
+    q.K = std::max(p.K, 0);
+    q.alpha = p.alpha;
+    q.beta = p.beta;
+    q.mode = p.mode;
+    q.tiles_m = (p.M + kBM - 1) / kBM;
+    q.tiles_n = (p.N + kBN - 1) / kBN;
+    q.tile_begin = tb;
+    tb += q.tiles_m * q.tiles_n;
+    if (q.K > 0 && bf16) {
+      q.a_mn = 0;
+      q.b_mn = 0;
+      // op(A) as (m, k) and op(B)^T as (n, k), both K-major.
+      const float* src[2] = {p.A, p.B};
+      const int lds[2] = {p.lda, p.ldb};
+      const int mnd[2] = {p.M, p.N};
+      const int kc[2] = {p.transA ? 1 : 0, p.transB ? 0 : 1};
+      const int keep[2] = {(p.mode & kTriAUpper) ? 1 : (p.mode & kTriALower) ? 2 : 0,
+                           (p.mode & kTriBUpper) ? 2 : (p.mode & kTriBLower) ? 1 : 0};
+      CUtensorMap* maps[2] = {q.a, q.b};
+      for (int o = 0; o < 2; ++o) {
+        const int ldk = pad8(q.K);
+        const size_t half = (size_t)ldk * mnd[o];  // bf16 elements per piece
+        __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(w);
+        SplitJob16& J = sp16.j[sp16.njobs++];
+        J.src = src[o];
+        J.lds = lds[o];
+        J.K = q.K;
+        J.MN = mnd[o];
+        J.ldk = ldk;
+        J.k_contig = kc[o];
+        J.keep = keep[o];
+        J.hi = base;
+        J.lo = base + ((half + 63) & ~size_t(63));
+        w += ((half + 63) & ~size_t(63));  // two BF16 pieces take the room of one FP32 copy
+        max_total = std::max<int>(max_total, (int)std::min<size_t>(half, 1u << 30));
+        if (!encode_operand_bf16(&maps[o][0], J.hi, q.K, mnd[o], ldk) ||
+            !encode_operand_bf16(&maps[o][1], J.lo, q.K, mnd[o], ldk))
+          return cudaErrorInvalidValue;
+      }
+    } else if (q.K > 0) {
+      const OperandShape sa = shape_a(p), sb = shape_b(p);
+      q.a_mn = sa.mn ? 1 : 0;
+      q.b_mn = sb.mn ? 1 : 0;
+      const OperandShape* shp[2] = {&sa, &sb};
+      const float* src[2] = {p.A, p.B};
+      const int lds[2] = {p.lda, p.ldb};
+      CUtensorMap* maps[2] = {q.a, q.b};
+      for (int o = 0; o < 2; ++o) {
+        const OperandShape& sh = *shp[o];
+        const int ldp = pad4(sh.rows);
+        const size_t half = up64((size_t)ldp * sh.cols);
+        SplitJob& J = sp.j[sp.njobs++];
+        J.src = src[o];
+        J.lds = lds[o];
+        J.rows = sh.rows;
+        J.cols = sh.cols;
+        J.ldp = ldp;
+        J.keep = sh.keep;
+        J.hi = w;
+        J.lo = w + half;
+        w += 2 * half;
+        max_total = std::max<int>(max_total, (int)std::min<size_t>((size_t)ldp * sh.cols, 1u << 30));
+        if (!encode_operand(&maps[o][0], J.hi, sh.rows, sh.cols, ldp, sh.mn) ||
+            !encode_operand(&maps[o][1], J.lo, sh.rows, sh.cols, ldp, sh.mn))
+          return cudaErrorInvalidValue;
+      }
+    }
+    ++used;
+  }
+  if (used == 0 || tb == 0) return cudaSuccess;
+  up.nprob = used;
+  up.passes = passes;
+  up.st = st;
+  up.limit_ns = limit_ns;
+  if (sp.njobs > 0) {
+    const int bx = (int)std::min<long>((max_total + 255) / 256, 148 * 4);
+    umma_split_kernel<kMax><<<dim3(std::max(bx, 1), sp.njobs), 256, 0, s>>>(sp);
+    note_launches();
+  }
+  if (sp16.njobs > 0) {
+    const int bx = (int)std::min<long>((max_total + 255) / 256, 148 * 4);
+    umma_split_bf16_kernel<kMax><<<dim3(std::max(bx, 1), sp16.njobs), 256, 0, s>>>(sp16);
+    note_launches();
+  }
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  auto kern = bf16 ? umma_gemm_kernel<true, kMax> : umma_gemm_kernel<false, kMax>;
+  if (dev < 0 || dev >= 64 || !smem_set[bf16][dev]) {
+    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (err != cudaSuccess) return err;
+    if (dev >= 0 && dev < 64) smem_set[bf16][dev] = true;
+  }
+  kern<<<tb, kThreads, kSmemBytes, s>>>(up);
+  note_launches();
+  return cudaGetLastError();
+}
+
+}  // namespace
+
 cudaError_t umma_gemm_group(const GemmDesc<float>* probs, int nprob, int passes, float* work, size_t work_elems,
                             DeviceStatus* st, uint64_t limit_ns, cudaStream_t s) {
   if (passes != 1 && passes != 3 && passes != 11 && passes != 13) return cudaErrorInvalidValue;
   const bool bf16 = passes > 10;
   if (bf16) passes -= 10;
-  for (int base = 0; base < nprob; base += kMaxProbs) {
-    const int cnt = std::min(kMaxProbs, nprob - base);
+  for (int base = 0, cnt; base < nprob; base += cnt) {
+    cnt = std::min(kFewProbs, nprob - base);
     if (umma_work_elems(probs + base, cnt) > work_elems) return cudaErrorInvalidValue;
-    UParams up;
-    memset(&up, 0, sizeof(up));
-    SplitParams sp;
-    memset(&sp, 0, sizeof(sp));
-    sp.passes = passes;
-    Split16Params sp16;
-    memset(&sp16, 0, sizeof(sp16));
-    sp16.pieces = passes == 3 ? 2 : 1;
-    float* w = work;
-    int tb = 0, used = 0, max_total = 0;
-    for (int i = 0; i < cnt; ++i) {
-      const GemmDesc<float>& p = probs[base + i];
-      if (p.M <= 0 || p.N <= 0) continue;
-      UProb& q = up.p[used];
-      q.C = p.C;
-      q.ldc = p.ldc;
-      q.M = p.M;
-      q.N = p.N;
-      q.K = std::max(p.K, 0);
-      q.alpha = p.alpha;
-      q.beta = p.beta;
-      q.mode = p.mode;
-      q.tiles_m = (p.M + kBM - 1) / kBM;
-      q.tiles_n = (p.N + kBN - 1) / kBN;
-      q.tile_begin = tb;
-      tb += q.tiles_m * q.tiles_n;
-      if (q.K > 0 && bf16) {
-        q.a_mn = 0;
-        q.b_mn = 0;
-        // op(A) as (m, k) and op(B)^T as (n, k), both K-major.
-        const float* src[2] = {p.A, p.B};
-        const int lds[2] = {p.lda, p.ldb};
-        const int mnd[2] = {p.M, p.N};
-        const int kc[2] = {p.transA ? 1 : 0, p.transB ? 0 : 1};
-        const int keep[2] = {(p.mode & kTriAUpper) ? 1 : (p.mode & kTriALower) ? 2 : 0,
-                             (p.mode & kTriBUpper) ? 2 : (p.mode & kTriBLower) ? 1 : 0};
-        CUtensorMap* maps[2] = {q.a, q.b};
-        for (int o = 0; o < 2; ++o) {
-          const int ldk = pad8(q.K);
-          const size_t half = (size_t)ldk * mnd[o];  // bf16 elements per piece
-          __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(w);
-          SplitJob16& J = sp16.j[sp16.njobs++];
-          J.src = src[o];
-          J.lds = lds[o];
-          J.K = q.K;
-          J.MN = mnd[o];
-          J.ldk = ldk;
-          J.k_contig = kc[o];
-          J.keep = keep[o];
-          J.hi = base;
-          J.lo = base + ((half + 63) & ~size_t(63));
-          w += ((half + 63) & ~size_t(63));  // two BF16 pieces take the room of one FP32 copy
-          max_total = std::max<int>(max_total, (int)std::min<size_t>(half, 1u << 30));
-          if (!encode_operand_bf16(&maps[o][0], J.hi, q.K, mnd[o], ldk) ||
-              !encode_operand_bf16(&maps[o][1], J.lo, q.K, mnd[o], ldk))
-            return cudaErrorInvalidValue;
-        }
-      } else if (q.K > 0) {
-        const OperandShape sa = shape_a(p), sb = shape_b(p);
-        q.a_mn = sa.mn ? 1 : 0;
-        q.b_mn = sb.mn ? 1 : 0;
-        const OperandShape* shp[2] = {&sa, &sb};
-        const float* src[2] = {p.A, p.B};
-        const int lds[2] = {p.lda, p.ldb};
-        CUtensorMap* maps[2] = {q.a, q.b};
-        for (int o = 0; o < 2; ++o) {
-          const OperandShape& sh = *shp[o];
-          const int ldp = pad4(sh.rows);
-          const size_t half = up64((size_t)ldp * sh.cols);
-          SplitJob& J = sp.j[sp.njobs++];
-          J.src = src[o];
-          J.lds = lds[o];
-          J.rows = sh.rows;
-          J.cols = sh.cols;
-          J.ldp = ldp;
-          J.keep = sh.keep;
-          J.hi = w;
-          J.lo = w + half;
-          w += 2 * half;
-          max_total = std::max<int>(max_total, (int)std::min<size_t>((size_t)ldp * sh.cols, 1u << 30));
-          if (!encode_operand(&maps[o][0], J.hi, sh.rows, sh.cols, ldp, sh.mn) ||
-              !encode_operand(&maps[o][1], J.lo, sh.rows, sh.cols, ldp, sh.mn))
-            return cudaErrorInvalidValue;
-        }
-      }
-      ++used;
-    }
-    if (used == 0 || tb == 0) continue;
-    up.nprob = used;
-    up.passes = passes;
-    up.st = st;
-    up.limit_ns = limit_ns;
-    if (sp.njobs > 0) {
-      const int bx = (int)std::min<long>((max_total + 255) / 256, 148 * 4);
-      umma_split_kernel<<<dim3(std::max(bx, 1), sp.njobs), 256, 0, s>>>(sp);
-      note_launches();
-    }
-    if (sp16.njobs > 0) {
-      const int bx = (int)std::min<long>((max_total + 255) / 256, 148 * 4);
-      umma_split_bf16_kernel<<<dim3(std::max(bx, 1), sp16.njobs), 256, 0, s>>>(sp16);
-      note_launches();
-    }
-    int dev = 0;
-    cudaError_t err = cudaGetDevice(&dev);
-    if (err != cudaSuccess) return err;
-    auto kern = bf16 ? umma_gemm_kernel<true> : umma_gemm_kernel<false>;
-    if (dev < 0 || dev >= 64 || !g_smem_set[bf16][dev]) {
-      err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-      if (err != cudaSuccess) return err;
-      if (dev >= 0 && dev < 64) g_smem_set[bf16][dev] = true;
-    }
-    kern<<<tb, kThreads, kSmemBytes, s>>>(up);
-    note_launches();
-    err = cudaGetLastError();
+    // As many problems as a launch and the workspace take.
+    while (cnt < kManyProbs && base + cnt < nprob && umma_work_elems(probs + base, cnt + 1) <= work_elems) ++cnt;
+    const cudaError_t err = cnt <= kFewProbs
+                                ? umma_launch<kFewProbs>(probs + base, cnt, passes, bf16, work, st, limit_ns, s)
+                                : umma_launch<kManyProbs>(probs + base, cnt, passes, bf16, work, st, limit_ns, s);
     if (err != cudaSuccess) return err;
   }
   return cudaSuccess;
