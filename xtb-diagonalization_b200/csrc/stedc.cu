@@ -315,8 +315,8 @@ __global__ void __launch_bounds__(1024) dc_deflate_kernel(DcBufs B, int nmerge) 
 #pragma unroll
     for (int t = 0; t < 4; ++t) cnt[t] += ty == t + 1;
   }
-  const Counts pre = block_exscan4(Counts{cnt[0] | (unsigned long long)cnt[1] << 32, cnt[2] | (unsigned long long)cnt[3] << 32},
-                                   s_scan, &tot);
+  const Counts mine{cnt[0] | (unsigned long long)cnt[1] << 32, cnt[2] | (unsigned long long)cnt[3] << 32};
+  const Counts pre = block_exscan4(mine, s_scan, &tot);
   const int c1 = (int)(unsigned)tot.a, c2 = (int)(tot.a >> 32), c3 = (int)(unsigned)tot.b, nd = (int)(tot.b >> 32);
   const int K = c1 + c2 + c3;
   int at1 = (int)(unsigned)pre.a, at2 = (int)(pre.a >> 32), at3 = (int)(unsigned)pre.b, atd = (int)(pre.b >> 32);
@@ -429,9 +429,10 @@ struct SecSums {
 template <int WPR>
 constexpr int kRootThreads = WPR == 0 ? 8 : 32 * WPR;
 
-// A root is solved by WPR warps together (one CTA of 32 WPR threads when WPR > 1) or by eight lanes: every sum runs over the poles
-// strided by the group's threads, then across its warps in warp order through shared memory (sh: 2 x 5 x WPR doubles,
-// alternating by `tog`, so one __syncthreads per sum; every thread receives the same value).  The groups of eight of a warp may diverge.
+// A root is solved by WPR warps together (one CTA of 32 WPR threads when WPR > 1) or by eight lanes: every sum runs over
+// the poles strided by the group's threads, then across its warps in warp order through shared memory (sh: 2 x 5 x WPR
+// doubles, alternating by `tog`, so one __syncthreads per sum; every thread receives the same value).  The groups of
+// eight of a warp may diverge.
 template <int WPR>
 __device__ __forceinline__ void group_sums(double* v, int cnt, double* sh, int& tog) {
   if constexpr (WPR == 0) {

@@ -43,10 +43,10 @@ constexpr int kBM = 128, kBN = 128, kBK = 32, kStages = 3, kThreads = 128;
 constexpr int kTileBytes = kBM * kBK * 4;          // one operand tile (A or B, hi or lo): 16 KB
 constexpr int kStageBytes = 4 * kTileBytes;        // A hi, A lo, B hi, B lo
 constexpr int kSmemBytes = kStages * kStageBytes + 1024;
-// Problems per launch.  The descriptors travel as kernel parameters (576 bytes per problem, 32 KB at most), so few problems
-// take the small form and the Gram matrices of a whole back-transformation (86 at n = 1788) two launches of the large
-// one instead of eleven (mixed solve at n = 1788: 8402 -> 8300 us; the stream that
-// forms X Q beside the divide and conquer ends 200 us earlier).
+// Problems per launch.  The descriptors travel as kernel parameters (576 bytes per problem, 32 KB at most), so few
+// problems take the small form and the Gram matrices of a whole back-transformation (86 at n = 1788) two launches of the
+// large one instead of eleven (mixed solve at n = 1788: 8402 -> 8300 us; the stream that forms X Q beside the divide and
+// conquer ends 200 us earlier).
 constexpr int kFewProbs = 8, kManyProbs = 48;
 constexpr uint32_t kTmemCols = 128;
 
