@@ -174,8 +174,8 @@ __device__ __forceinline__ void warp_row_sums(float (&acc)[kRowChunk], float* ou
   if ((lane & 3) == 0 && (ROWS == 8 || h2 == false)) out[ROWS == 8 ? lane >> 2 : lane >> 3] = r;
 }
 
-// One row chunk of the pass over the first JA column pairs: ROWS register rows, or ROWS rows of shared (global) memory
-// with the last pair's columns tested against k.  Straight-line code, so that the rows' dependent chains interleave (a
+// One row chunk of the pass over the first JA column pairs: ROWS register rows, or ROWS rows of shared (global) memory,
+// whose pairs from FULL on are tested against k (the pairs before lie below k in every thread).  Straight-line code, so that the rows' dependent chains interleave (a
 // branch per row and pair left every chain's latency exposed: 5700 cycles instead of 2000 for 13 rows of 1788).
 template <int ROWS, int JA, int CPT, typename T>
 __device__ __forceinline__ void pass_registers(T (*ra)[CPT], const Pair<T>* vy, T tau, T half, const T* wk, const T* vk,
@@ -199,19 +199,19 @@ __device__ __forceinline__ void pass_registers(T (*ra)[CPT], const Pair<T>* vy, 
   }
 }
 
-template <int ROWS, int JA, int NT, typename T>
+template <int ROWS, int JA, int FULL, int NT, typename T>
 __device__ __forceinline__ void pass_memory(T* row0, size_t ldr, int k, const Pair<T>* vy, T tau, T half, const T* wk,
                                             const T* vk, const T* xs, T* acc) {
   // Every load before the first store: the stores could alias the loads for all the compiler knows.
   Pair<T> e[ROWS][JA];
   const int c0 = 2 * (int)threadIdx.x;
-  const bool in = c0 + 2 * (JA - 1) * NT < k;  // the last pair's columns
+  auto in = [&](int j) { return j < FULL || c0 + 2 * j * NT < k; };
 #pragma unroll
   for (int q = 0; q < ROWS; ++q)
 #pragma unroll
     for (int j = 0; j < JA; ++j) {
-      if (j == JA - 1) e[q][j] = Pair<T>{T(0), T(0)};
-      if (j < JA - 1 || in) e[q][j] = *reinterpret_cast<const Pair<T>*>(row0 + q * ldr + c0 + 2 * j * NT);
+      if (j >= FULL) e[q][j] = Pair<T>{T(0), T(0)};
+      if (in(j)) e[q][j] = *reinterpret_cast<const Pair<T>*>(row0 + q * ldr + c0 + 2 * j * NT);
     }
   T vr[ROWS], wr[ROWS];
 #pragma unroll
@@ -232,7 +232,7 @@ __device__ __forceinline__ void pass_memory(T* row0, size_t ldr, int k, const Pa
   for (int q = 0; q < ROWS; ++q)
 #pragma unroll
     for (int j = 0; j < JA; ++j)
-      if (j < JA - 1 || in) *reinterpret_cast<Pair<T>*>(row0 + q * ldr + c0 + 2 * j * NT) = e[q][j];
+      if (in(j)) *reinterpret_cast<Pair<T>*>(row0 + q * ldr + c0 + 2 * j * NT) = e[q][j];
 }
 
 // kUpperInPlace: the variant that reads the upper triangle of p.afull (== p.aout) in place instead of a full
@@ -342,8 +342,10 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
     if (2 * NT * (ja - 1) >= k) --ja;
 
     // One column, over the first JA column pairs of every thread (the others lie beyond k).
+    // Pairs wholly below k: all but the last, unless this code serves several counts of active pairs (CP 8 and more: 1 to
+    // 4, and 5 to CP), where a pair past the active ones would lie in the next row.
     auto step = [&](auto JA) {
-      constexpr int J = decltype(JA)::value, E = 2 * J;
+      constexpr int J = decltype(JA)::value, E = 2 * J, FULL = CP <= 4 ? J - 1 : J > 4 ? 4 : 0;
       // ||x||^2 of x = A(0:k-2, k): per-warp partials, summed after the pass's __syncthreads.
       T part;
       {
@@ -380,11 +382,11 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
         T* row = rows + (size_t)(q0 - RR) * ldr;
         const Pair<T>* o = vy + q0;
         // Rows in pairs, so at most one row beyond nq (its storage exists: R is even); sums beyond nq are not read.
-        pass_memory<2, J, NT, T>(row, ldr, k, o, tau_prev, half_prev, wk, vk, xs, acc);
-        if (rem > 2) pass_memory<2, J, NT, T>(row + 2 * ldr, ldr, k, o + 2, tau_prev, half_prev, wk, vk, xs, acc + 2);
+        pass_memory<2, J, FULL, NT, T>(row, ldr, k, o, tau_prev, half_prev, wk, vk, xs, acc);
+        if (rem > 2) pass_memory<2, J, FULL, NT, T>(row + 2 * ldr, ldr, k, o + 2, tau_prev, half_prev, wk, vk, xs, acc + 2);
         if (rem > 4) {
-          pass_memory<2, J, NT, T>(row + 4 * ldr, ldr, k, o + 4, tau_prev, half_prev, wk, vk, xs, acc + 4);
-          if (rem > 6) pass_memory<2, J, NT, T>(row + 6 * ldr, ldr, k, o + 6, tau_prev, half_prev, wk, vk, xs, acc + 6);
+          pass_memory<2, J, FULL, NT, T>(row + 4 * ldr, ldr, k, o + 4, tau_prev, half_prev, wk, vk, xs, acc + 4);
+          if (rem > 6) pass_memory<2, J, FULL, NT, T>(row + 6 * ldr, ldr, k, o + 6, tau_prev, half_prev, wk, vk, xs, acc + 6);
           warp_row_sums<8>(acc, red + warp * (R + 8) + q0);
         } else {
           warp_row_sums<4>(acc, red + warp * (R + 8) + q0);
