@@ -342,10 +342,10 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
     if (2 * NT * (ja - 1) >= k) --ja;
 
     // One column, over the first JA column pairs of every thread (the others lie beyond k).
-    // Pairs wholly below k: all but the last, unless this code serves several counts of active pairs (CP 8 and more: 1 to
-    // 4, and 5 to CP), where a pair past the active ones would lie in the next row.
+    // FULL pairs lie wholly below k: all but the last, unless this code serves several counts of active pairs (CP 8: 1 to
+    // 4, and 5 to 8), where a pair past the active ones would lie in the next row.
     auto step = [&](auto JA) {
-      constexpr int J = decltype(JA)::value, E = 2 * J, FULL = CP <= 4 ? J - 1 : J > 4 ? 4 : 0;
+      constexpr int J = decltype(JA)::value, E = 2 * J, FULL = CP <= 4 ? J - 1 : 0;
       // ||x||^2 of x = A(0:k-2, k): per-warp partials, summed after the pass's __syncthreads.
       T part;
       {
@@ -381,12 +381,24 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
         const int rem = nq - q0;
         T* row = rows + (size_t)(q0 - RR) * ldr;
         const Pair<T>* o = vy + q0;
-        // Rows in pairs, so at most one row beyond nq (its storage exists: R is even); sums beyond nq are not read.
-        pass_memory<2, J, FULL, NT, T>(row, ldr, k, o, tau_prev, half_prev, wk, vk, xs, acc);
-        if (rem > 2) pass_memory<2, J, FULL, NT, T>(row + 2 * ldr, ldr, k, o + 2, tau_prev, half_prev, wk, vk, xs, acc + 2);
+        // Rows in pairs, so at most one row beyond nq (its storage exists: R is even); sums beyond nq are not read.  Beside
+        // more than eight columns' x, v and w the registers hold one column pair of two rows: all eight pairs at once
+        // (n > 8192, FP64) spilled: n = 9500 2.02 s, 13000 5.64 s; one at a time 1.57 and 3.65.
+        auto pair = [&](int i) {
+          if constexpr (J <= 4) {
+            pass_memory<2, J, FULL, NT, T>(row + i * ldr, ldr, k, o + i, tau_prev, half_prev, wk, vk, xs, acc + i);
+          } else {
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+              pass_memory<2, 1, 0, NT, T>(row + i * ldr + 2 * j * NT, ldr, k - 2 * j * NT, o + i, tau_prev, half_prev,
+                                          wk + 2 * j, vk + 2 * j, xs + 2 * j, acc + i);
+          }
+        };
+        pair(0);
+        if (rem > 2) pair(2);
         if (rem > 4) {
-          pass_memory<2, J, FULL, NT, T>(row + 4 * ldr, ldr, k, o + 4, tau_prev, half_prev, wk, vk, xs, acc + 4);
-          if (rem > 6) pass_memory<2, J, FULL, NT, T>(row + 6 * ldr, ldr, k, o + 6, tau_prev, half_prev, wk, vk, xs, acc + 6);
+          pair(4);
+          if (rem > 6) pair(6);
           warp_row_sums<8>(acc, red + warp * (R + 8) + q0);
         } else {
           warp_row_sums<4>(acc, red + warp * (R + 8) + q0);
