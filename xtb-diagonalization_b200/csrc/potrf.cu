@@ -41,35 +41,46 @@ struct PotrfParams {
 };
 
 constexpr int kLeafLd = NB + 4;  // 4 (mod 16): fragment loads of a half warp hit 16 distinct 8-byte banks
-constexpr size_t kLeafElems = (size_t)NB * kLeafLd + NB + 4;  // rows, U(k, k), row counter and flag
+constexpr size_t kLeafElems = (size_t)NB * kLeafLd + NB + 4;  // rows, pivots, row counter and flag
 constexpr size_t kSmemBytes = (tile::smem_elems<double>() + kLeafElems) * sizeof(double);
 static_assert((size_t)NB * kLeafLd <= tile::smem_elems<double>(), "the panel fits the tile pipeline's region");
 
 // 1 / sqrt(d) for d > 0 without a branch, so that the pivot chain interleaves with the row updates: the hardware's
 // approximation y and one third-order step, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - d y^2 (the series of (1 - e)^(-1/2); the
-// approximation's error cubed is far below the last bit).  The approximation flushes subnormal arguments, so small d
-// are scaled by 2^200 first.
+// approximation's error cubed is far below the last bit).  e comes from the exact product d y = p + pl: with p alone its
+// rounding was as large as the result's own (0.99 ulp instead of 0.52).  The approximation flushes subnormal arguments,
+// so small d are scaled by 2^200 first.
 __device__ __forceinline__ double pivot_rsqrt(double d) {
   const bool small = d < 1e-250;
   const double ds = small ? d * 0x1p200 : d;
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(ds));
-  const double e = fma(-ds * y, y, 1.0);
+  const double p = ds * y, pl = fma(ds, y, -p);
+  const double e = fma(-pl, y, fma(-p, y, 1.0));
   const double r = fma(y * e, fma(0.375, e, 0.5), y);
   return small ? r * 0x1p100 : r;
 }
+// sqrt(d) from r = pivot_rsqrt(d): one Newton step on d r, whose residual is exact except where it would be subnormal.
+__device__ __forceinline__ double pivot_sqrt(double d, double r) {
+  const double s = d * r;
+  return d < 1e-280 ? s : fma(fma(-s, s, d), 0.5 * r, s);
+}
 
-// Elimination steps k = 16 b .. 16 b + 15 of the leaf (see leaf_factor_invert) on the 16 rows of one warp: its owner,
-// warp b, leaves the final rows in `rows` and counts them in *done, two at a time; the warps below follow.  Both are
-// rolled loops of about a hundred instructions: unrolled over the 64 steps the code, run once per leaf, was bound by
-// instruction fetch (twice the time).
 // The pivot state of the owner warp, the same in every lane: d = M(k, k), r = 1 / sqrt(d), and the two values the next
 // pivot follows from, a = M(k, k+1) and b = M(k+1, k+1): d' = b - (a r)^2 needs no shuffle once r is known.
 struct LeafPivot {
   double d, r, a, b;
-  int bad;  // first pivot of this block that is not > 0
+  double x0, x1;  // the pivot row's entries in this lane's columns
+  int bad;        // first pivot of this block that is not > 0
 };
 
+// Elimination steps k = 16 b .. 16 b + 15 of the leaf (see leaf_factor_invert) on the 16 rows of one warp: its owner,
+// warp b, leaves the final rows in `rows` and counts them in *done, two at a time; the warps below follow.  Both are
+// rolled loops of about a hundred instructions: unrolled over the 64 steps the code, run once per leaf, was bound by
+// instruction fetch (twice the time).  m holds the sum of the products subtracted so far; the block's own row stays in
+// `rows` and joins when it becomes the pivot row, so that an entry is rounded once at the block's magnitude.  With the
+// products subtracted from the entry one by one, U^T U was three times as far from S (n = 130: 1.2e-15 against 4.1e-16,
+// S(k, k) about 2) and the whole factorization 2 % faster.
 // kSecond: column k lies in the lanes' second column.  Q0: first of the 16 steps; ROWS: rows below the pivot that may
 // still be unfinished (15 in the first eight steps, 7 in the last eight).
 template <bool kSecond, int Q0, int ROWS>
@@ -82,13 +93,16 @@ __device__ __forceinline__ void leaf_own_steps(double (&m)[16][2], LeafPivot& v,
     const int k = 16 * blk + q;
     const bool at = lane == l0 + q;
     const double r = v.r, u1 = v.a * r;
+    // The block's own entries of the next row and of the pivot after it (past the last row: unused).
+    const int k1 = min(k + 1, NB - 1), k2 = min(k + 2, NB - 1);
+    const double n0 = rows[k1 * kLeafLd + lane], n1 = rows[k1 * kLeafLd + lane + 32], nb = rows[k2 * kLeafLd + k2];
     v.bad = (!(v.d > 0.0) && v.bad < 0) ? k : v.bad;
     // U(k, :) right of k, W(k, :) from k to the left.
-    const double p0 = (!kSecond && at) ? r : m[0][0] * r, p1 = (kSecond && at) ? r : m[0][1] * r;
+    const double p0 = (!kSecond && at) ? r : v.x0 * r, p1 = (kSecond && at) ? r : v.x1 * r;
     double* row = rows + k * kLeafLd;
     row[lane] = p0;
     row[lane + 32] = p1;
-    if (lane == 0) diag[k] = v.d * r;
+    if (lane == 0) diag[k] = v.d;
     v.d = fma(-u1, u1, v.b);
     v.r = pivot_rsqrt(v.d);  // beside the row updates
 #pragma unroll
@@ -97,9 +111,13 @@ __device__ __forceinline__ void leaf_own_steps(double (&m)[16][2], LeafPivot& v,
       const double u = i == 1 ? u1 : __shfl_sync(0xffffffffu, kSecond ? p1 : p0, l0 + q + i);
       m[i - 1][0] = fma(-u, p0, (!kSecond && at) ? 0.0 : m[i][0]);  // column k becomes -U(k, row) W(k, k)
       m[i - 1][1] = fma(-u, p1, (kSecond && at) ? 0.0 : m[i][1]);
+      if (i == 1) {
+        v.x0 = n0 + m[0][0];
+        v.x1 = n1 + m[0][1];
+      }
       if (i == 3) {
-        v.a = __shfl_sync(0xffffffffu, kSecond ? m[0][1] : m[0][0], l0 + q + 2);
-        v.b = __shfl_sync(0xffffffffu, kSecond ? m[1][1] : m[1][0], l0 + q + 2);
+        v.a = __shfl_sync(0xffffffffu, kSecond ? v.x1 : v.x0, l0 + q + 2);
+        v.b = nb + __shfl_sync(0xffffffffu, kSecond ? m[1][1] : m[1][0], l0 + q + 2);
       }
     }
     if (q & 1) {
@@ -114,10 +132,13 @@ template <bool kSecond>
 __device__ __forceinline__ void leaf_own_block(double (&m)[16][2], int blk, double* rows, double* diag,
                                                volatile int* done, int* s_bad, int lane) {
   const int l0 = (16 * blk) & 31;
+  const double* row = rows + 16 * blk * kLeafLd;
   LeafPivot v;
-  v.d = __shfl_sync(0xffffffffu, kSecond ? m[0][1] : m[0][0], l0);
-  v.a = __shfl_sync(0xffffffffu, kSecond ? m[0][1] : m[0][0], l0 + 1);
-  v.b = __shfl_sync(0xffffffffu, kSecond ? m[1][1] : m[1][0], l0 + 1);
+  v.x0 = row[lane] + m[0][0];
+  v.x1 = row[lane + 32] + m[0][1];
+  v.d = __shfl_sync(0xffffffffu, kSecond ? v.x1 : v.x0, l0);
+  v.a = __shfl_sync(0xffffffffu, kSecond ? v.x1 : v.x0, l0 + 1);
+  v.b = row[16 * blk + 1 + kLeafLd] + __shfl_sync(0xffffffffu, kSecond ? m[1][1] : m[1][0], l0 + 1);
   v.r = pivot_rsqrt(v.d);
   v.bad = -1;
   leaf_own_steps<kSecond, 0, 15>(m, v, blk, rows, diag, done, lane);
@@ -165,14 +186,15 @@ __device__ __forceinline__ void leaf_follow_steps(double (&m)[16][2], int b, con
 // diagonal the rows then grow W = U^-T, which takes the place of A's lower triangle (at step k column k becomes
 // -U(k, i) W(k, k)), so the inverse costs no further step.  The owner warp runs down its 16 rows by shuffles alone,
 // leaving each final row in shared memory; the warps below follow it at their own pace (a row counter, no block
-// barrier).  One block alone (with its panel update): 39 k cycles, where panels of 8 columns with block barriers and a
-// separate block-wise inverse took 57 k; potrf + inverse n = 130 148 -> 118 us, 619 514 -> 420, 1788 1.41 -> 1.2 ms.
+// barrier).  One block alone (with its panel update): about 40 k cycles, where panels of 8 columns with block barriers and
+// a separate block-wise inverse took 57 k; potrf + inverse n = 130 152 -> 122 us, 619 493 -> 407, 1788 1.40 -> 1.05 ms (of
+// which the tiles of the trailing update, gemm_tile, gave a part).
 // With a panel (the kp x nb block row U(j0 - kp : j0, j0 : j0 + nb), ld lda), the block's trailing update
 // A -= P^T P runs first, by matrix instructions (gsm: the tile pipeline's region, free while the leaf runs, holds P).
 __device__ bool leaf_factor_invert(const double* panel, int kp, double* a, int lda, double* x, int ldx, int j0,
                                    int nb, DeviceStatus* st, double* smem, double* gsm) {
   double* rows = smem;                      // [64][kLeafLd]
-  double* diag = rows + NB * kLeafLd;       // U(k, k)
+  double* diag = rows + NB * kLeafLd;       // the pivots, then U(k, k)
   int* s_bad = reinterpret_cast<int*>(diag + NB);
   volatile int* done = s_bad + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -221,18 +243,15 @@ __device__ bool leaf_factor_invert(const double* panel, int kp, double* a, int l
       const int r = 8 * (first ? rows0 : rows1) + cr, c = 8 * (first ? rows0 + t : rows1 + t - (8 - rows0)) + 2 * kr;
       double2* dst = reinterpret_cast<double2*>(rows + r * kLeafLd + c);
       double2 v = *dst;
-      v.x -= acc[t][0];
-      v.y -= acc[t][1];
+      v.x -= r <= c ? acc[t][0] : 0.0;  // below the diagonal the rows stay zero: W joins them there
+      v.y -= r <= c + 1 ? acc[t][1] : 0.0;
       *dst = v;
     }
     __syncthreads();
   }
   double m[16][2];
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) m[i][j] = rows[(16 * warp + i) * kLeafLd + lane + 32 * j];
-  __syncthreads();  // every row has been read before the first final row is written
+  for (int i = 0; i < 16; ++i) m[i][0] = m[i][1] = 0.0;
 #pragma unroll 1
   for (int b = 0; b < warp; ++b) {
     if (b < 2) leaf_follow_steps<false>(m, b, rows, done, warp, lane);
@@ -246,6 +265,8 @@ __device__ bool leaf_factor_invert(const double* panel, int kp, double* a, int l
     __syncthreads();
     return false;
   }
+  if (tid < NB) diag[tid] = pivot_sqrt(diag[tid], rows[tid * kLeafLd + tid]);
+  __syncthreads();
 #pragma unroll 8
   for (int idx = tid; idx < NB * NB; idx += kThreads) {
     const int r = idx % NB, c = idx / NB;
