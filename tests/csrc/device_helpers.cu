@@ -1,0 +1,33 @@
+// Kernels that call single device helpers of the library, for tests/test_gpu_device_helpers.py.
+#include "common.cuh"
+
+using namespace xtbeig;
+
+__global__ void wait_kernel(int raise_to, int want, uint64_t limit_ns, DeviceStatus* st, int* result) {
+  __shared__ int count;
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    result[threadIdx.x] = wait_count(&count, want, st, limit_ns, 5) ? 1 : 0;
+  } else if (threadIdx.x == 32) {
+    *(volatile int*)&count = raise_to;
+  }
+}
+
+// One warp waits for a counter that another raises to raise_to.  Returns the CUDA error.
+extern "C" int run_wait(int raise_to, int want, long long limit_ns, int* status, int* result) {
+  DeviceStatus* st = nullptr;
+  int* r = nullptr;
+  cudaError_t err = cudaMalloc(&st, sizeof(DeviceStatus));
+  if (err == cudaSuccess) err = cudaMalloc(&r, 32 * sizeof(int));
+  if (err == cudaSuccess) err = cudaMemset(st, 0, sizeof(DeviceStatus));
+  if (err == cudaSuccess) {
+    wait_kernel<<<1, 64>>>(raise_to, want, (uint64_t)limit_ns, st, r);
+    err = cudaDeviceSynchronize();
+  }
+  if (err == cudaSuccess) err = cudaMemcpy(status, st, sizeof(DeviceStatus), cudaMemcpyDeviceToHost);
+  if (err == cudaSuccess) err = cudaMemcpy(result, r, 32 * sizeof(int), cudaMemcpyDeviceToHost);
+  cudaFree(st);
+  cudaFree(r);
+  return (int)err;
+}

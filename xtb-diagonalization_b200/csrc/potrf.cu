@@ -148,14 +148,14 @@ __device__ __forceinline__ void leaf_own_block(double (&m)[16][2], int blk, doub
 
 template <bool kSecond>
 __device__ __forceinline__ void leaf_follow_steps(double (&m)[16][2], int b, const double* rows, const volatile int* done,
-                                                  int warp, int lane) {
+                                                  int warp, int lane, DeviceStatus* st, uint64_t limit_ns, bool& waits) {
 #pragma unroll 1
   for (int q = 0; q < 16; ++q) {
     const int k = 16 * b + q;
     if ((q & 1) == 0) {
-      // The owner never waits for this warp, so the wait ends; the count only keeps it bounded.
-      for (int spin = 0; *done < k + 2 && spin < (1 << 24); ++spin) {
-      }
+      // The owner never waits for this warp, so the wait ends.  One that ran out of time has set the status, which the
+      // next grid barrier returns on; the rows are then read as they are, without another wait.
+      waits = waits && wait_count(done, k + 2, st, limit_ns, k);
       __threadfence_block();
     }
     const bool at = lane == (k & 31);
@@ -192,7 +192,7 @@ __device__ __forceinline__ void leaf_follow_steps(double (&m)[16][2], int b, con
 // With a panel (the kp x nb block row U(j0 - kp : j0, j0 : j0 + nb), ld lda), the block's trailing update
 // A -= P^T P runs first, by matrix instructions (gsm: the tile pipeline's region, free while the leaf runs, holds P).
 __device__ bool leaf_factor_invert(const double* panel, int kp, double* a, int lda, double* x, int ldx, int j0,
-                                   int nb, DeviceStatus* st, double* smem, double* gsm) {
+                                   int nb, DeviceStatus* st, uint64_t limit_ns, double* smem, double* gsm) {
   double* rows = smem;                      // [64][kLeafLd]
   double* diag = rows + NB * kLeafLd;       // the pivots, then U(k, k)
   int* s_bad = reinterpret_cast<int*>(diag + NB);
@@ -252,10 +252,11 @@ __device__ bool leaf_factor_invert(const double* panel, int kp, double* a, int l
   double m[16][2];
 #pragma unroll
   for (int i = 0; i < 16; ++i) m[i][0] = m[i][1] = 0.0;
+  bool waits = true;  // no wait has run out
 #pragma unroll 1
   for (int b = 0; b < warp; ++b) {
-    if (b < 2) leaf_follow_steps<false>(m, b, rows, done, warp, lane);
-    else leaf_follow_steps<true>(m, b, rows, done, warp, lane);
+    if (b < 2) leaf_follow_steps<false>(m, b, rows, done, warp, lane, st, limit_ns, waits);
+    else leaf_follow_steps<true>(m, b, rows, done, warp, lane, st, limit_ns, waits);
   }
   if (warp < 2) leaf_own_block<false>(m, warp, rows, diag, done, s_bad, lane);
   else leaf_own_block<true>(m, warp, rows, diag, done, s_bad, lane);
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) potrf_persistent_kernel(PotrfPara
   if (ld_volatile_i32(&p.st->code) != 0) return;
   auto bsize = [&](int b) { return min(NB, n - b * NB); };
 
-  if (cta == 0) leaf_factor_invert(nullptr, 0, a, lda, x, ldx, 0, bsize(0), p.st, lsm, gsm);
+  if (cta == 0) leaf_factor_invert(nullptr, 0, a, lda, x, ldx, 0, bsize(0), p.st, p.limit_ns, lsm, gsm);
   if (!group_barrier(p.counter, (unsigned)G, epoch, p.st, p.limit_ns)) return;
   if (ld_volatile_i32(&p.st->code) != 0) return;
 
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1) potrf_persistent_kernel(PotrfPara
     const int m = nt - j - 1;
     if (cta == 0) {
       const int r0 = (j + 1) * NB;
-      leaf_factor_invert(a + j0 + (size_t)r0 * lda, nbj, a, lda, x, ldx, r0, bsize(j + 1), p.st, lsm, gsm);
+      leaf_factor_invert(a + j0 + (size_t)r0 * lda, nbj, a, lda, x, ldx, r0, bsize(j + 1), p.st, p.limit_ns, lsm, gsm);
     }
     const int ntile = m * (m + 1) / 2 - 1;  // upper tiles of the m x m trailing block, except (j+1, j+1)
     const int workers = G > 1 ? G - 1 : 1;
