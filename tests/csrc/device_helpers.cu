@@ -31,3 +31,17 @@ extern "C" int run_wait(int raise_to, int want, long long limit_ns, int* status,
   cudaFree(r);
   return (int)err;
 }
+
+__global__ void divide_kernel(int n, const double* a, const double* x, double* rcp, double* quot, double* plain) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  rcp[i] = rcp_normal(x[i]);
+  quot[i] = div_normal(a[i], x[i]);
+  plain[i] = a[i] / x[i];
+}
+
+// 1 / x, a / x and the compiler's a / x for n pairs in device memory.
+extern "C" int run_divide(int n, const double* a, const double* x, double* rcp, double* quot, double* plain) {
+  divide_kernel<<<(n + 255) / 256, 256>>>(n, a, x, rcp, quot, plain);
+  return (int)cudaDeviceSynchronize();
+}

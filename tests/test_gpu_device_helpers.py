@@ -32,3 +32,34 @@ def test_wait_count(helpers, raise_to, want, ends):
     assert err == 0
     assert np.array_equal(result, np.full(32, int(ends)))
     assert list(status[:3]) == ([0, 0, 0] if ends else [1, 0, 5])
+
+
+@pytest.mark.parametrize("case", ["unit", "secular", "wide", "near_powers", "negative"])
+def test_branch_free_division(helpers, case):
+    """rcp_normal and div_normal against extended precision: half an ulp for the last rounding, and a hundredth for what
+    precedes it (the cube of an approximation good to about 2^-20, and the residual's own correction).  Against the
+    compiler's division, which rounds once: at most the neighbouring value."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    n = 1 << 18
+    a, x = rng.uniform(1, 2, n), rng.uniform(1, 2, n)
+    if case == "secular":  # z^2 over differences of poles
+        a, x = 10.0 ** rng.uniform(-32, 0, n), 10.0 ** rng.uniform(-31, 0.3, n)
+    elif case == "wide":
+        a, x = np.ldexp(a, rng.integers(-400, 400, n)), np.ldexp(x, rng.integers(-400, 400, n))
+    elif case == "near_powers":
+        a = np.ldexp(1.0 + rng.integers(-64, 65, n) * 2.0**-52, rng.integers(-3, 4, n))
+        x = np.ldexp(1.0 + rng.integers(-64, 65, n) * 2.0**-52, rng.integers(-3, 4, n))
+    elif case == "negative":
+        a, x = a * rng.choice([-1, 1], n), -x
+    dev = [torch.from_numpy(v).cuda() for v in (a, x)] + [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    assert helpers.run_divide(n, *[ctypes.c_void_p(v.data_ptr()) for v in dev]) == 0
+    rcp, quot, plain = (v.cpu().numpy() for v in dev[2:])
+    al, xl = a.astype(np.longdouble), x.astype(np.longdouble)
+    for got, exact in ((rcp, 1 / xl), (quot, al / xl)):
+        # ulps of the exact value's binade (frexp: spacing on the lower side of a power of two is half as wide)
+        ulp = np.ldexp(np.longdouble(1), np.frexp(exact)[1] - 53)
+        assert (np.abs(got.astype(np.longdouble) - exact) / ulp).max() < 0.51
+    assert np.abs(quot.view(np.int64) - plain.view(np.int64)).max() <= 1

@@ -403,21 +403,8 @@ __global__ void dc_gather_kernel(DcBufs B) {
 
 // ------------------------------------------------------------------------------------------------ secular equation
 
-// 1 / x and a / x without a branch, so that the divisions of a loop overlap (the compiler's division branches to a slow
-// path, which left every one's latency of about 150 cycles exposed: a thread's 13 poles took 2300 cycles per evaluation).
-// The hardware's approximation, one third-order Newton step, y (1 + h + h^2) with h = 1 - x y, and for the quotient
-// Markstein's residual correction (IA-64 and Elementary Functions, 2000); either rounds once at the end.  x is normal: the
-// differences here are at least about 1e-31 of the scaled spectrum, and other values give a NaN, as bad input does.
-__device__ __forceinline__ double rcp_normal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = fma(-x, y, 1.0);
-  return fma(y, fma(h, h, h), y);
-}
-__device__ __forceinline__ double div_normal(double a, double x) {
-  const double y = rcp_normal(x), q = a * y;
-  return fma(fma(-q, x, a), y, q);
-}
+// The divisions below are common.cuh's rcp_normal and div_normal: their divisors, differences of poles and roots, are at
+// least about 1e-31 of the scaled spectrum, and bad input gives a NaN, as it would by any division.
 
 // Sums over the poles left of the root (psi <= 0), right of it (phi >= 0) and their derivatives; the sum of the terms'
 // absolute values is phi - psi.
