@@ -1,5 +1,7 @@
-// Kernels that call single device helpers of the library, for tests/test_gpu_device_helpers.py.
+// Kernels that call single device helpers of the library, and calls of its internal stages, for
+// tests/test_gpu_device_helpers.py.
 #include "common.cuh"
+#include "kernels.h"
 
 using namespace xtbeig;
 
@@ -44,4 +46,25 @@ __global__ void divide_kernel(int n, const double* a, const double* x, double* r
 extern "C" int run_divide(int n, const double* a, const double* x, double* rcp, double* quot, double* plain) {
   divide_kernel<<<(n + 255) / 256, 256>>>(n, a, x, rcp, quot, plain);
   return (int)cudaDeviceSynchronize();
+}
+
+// The divide and conquer stage on device buffers d (n), e (n - 1), z (ldz x n), with a status word that starts at `code`.
+extern "C" int run_stedc(int n, double* d, double* e, double* z, int ldz, int m_cols, int leaf, int code, int* status) {
+  void *work = nullptr, *plan = nullptr, *stage = nullptr;
+  DeviceStatus* st = nullptr;
+  const size_t wb = stedc_work_bytes(n), sb = (size_t)40 * n * sizeof(int) + 4 * (n + 8) * sizeof(GemmDesc<double>) + 4096;
+  const DeviceStatus start{code, 0, 0, 0};
+  cudaError_t err = cudaMalloc(&work, wb);
+  if (err == cudaSuccess) err = cudaMalloc(&plan, stedc_plan_bytes(n));
+  if (err == cudaSuccess) err = cudaMallocHost(&stage, sb);
+  if (err == cudaSuccess) err = cudaMalloc(&st, sizeof(start));
+  if (err == cudaSuccess) err = cudaMemcpy(st, &start, sizeof(start), cudaMemcpyHostToDevice);
+  if (err == cudaSuccess) err = stedc_device(n, d, e, z, ldz, work, wb, plan, true, stage, sb, st, nullptr, m_cols, leaf);
+  if (err == cudaSuccess) err = cudaDeviceSynchronize();
+  if (err == cudaSuccess) err = cudaMemcpy(status, st, sizeof(start), cudaMemcpyDeviceToHost);
+  cudaFree(st);
+  cudaFreeHost(stage);
+  cudaFree(plan);
+  cudaFree(work);
+  return (int)err;
 }

@@ -1,4 +1,4 @@
-"""Device helpers of csrc/common.cuh, called alone through the kernels of tests/csrc/device_helpers.cu."""
+"""Device helpers of csrc/common.cuh and internal stages, called alone through tests/csrc/device_helpers.cu."""
 import ctypes
 import importlib.util
 import os
@@ -19,7 +19,8 @@ def helpers(tmp_path_factory):
     spec.loader.exec_module(build)
     src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc", "device_helpers.cu")
     out = str(tmp_path_factory.mktemp("helpers") / "device_helpers.so")
-    subprocess.run([build.nvcc()] + build.ARCH + build.FLAGS + ["-I", build.CSRC, "-shared", "-o", out, src], check=True)
+    subprocess.run([build.nvcc()] + build.ARCH + build.FLAGS + ["-I", build.CSRC, "-shared", "-o", out, src, build.LIB,
+                                                                "-Xlinker", "-rpath=" + PKG], check=True)
     return ctypes.CDLL(out)
 
 
@@ -63,3 +64,35 @@ def test_branch_free_division(helpers, case):
         ulp = np.ldexp(np.longdouble(1), np.frexp(exact)[1] - 53)
         assert (np.abs(got.astype(np.longdouble) - exact) / ulp).max() < 0.51
     assert np.abs(quot.view(np.int64) - plain.view(np.int64)).max() <= 1
+
+
+def _stedc(helpers, n, m_cols, code):
+    import torch
+
+    from oracle import inputs
+
+    d, e = inputs.random_tridiagonal(n, 4100 + n)
+    dd, de = torch.from_numpy(d).cuda(), torch.from_numpy(np.append(e, 0.0)).cuda()
+    z = torch.full((n, n), 7.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    status = np.zeros(4, np.int32)
+    assert helpers.run_stedc(n, *[ctypes.c_void_p(v.data_ptr()) for v in (dd, de, z)], n, m_cols, 16, code,
+                             status.ctypes.data_as(ctypes.c_void_p)) == 0
+    return d, e, dd.cpu().numpy(), z.cpu().numpy().T, status[0]
+
+
+@pytest.mark.parametrize("n,m_cols", [(5, 1), (9, 8), (40, 3), (64, 63), (100, 30)])
+def test_stedc_writes_only_the_wanted_vectors(helpers, n, m_cols):
+    d, e, w, z, code = _stedc(helpers, n, m_cols, 0)
+    assert code == 0
+    t = np.diag(d) + np.diag(e, 1) + np.diag(e, -1)
+    np.testing.assert_allclose(w, np.linalg.eigvalsh(t), rtol=0, atol=5e-14 * n)
+    assert np.abs(t @ z[:, :m_cols] - z[:, :m_cols] * w[:m_cols]).max() < 1e-13 * n
+    assert np.all(z[:, m_cols:] == 7.0)
+
+
+@pytest.mark.parametrize("n", [5, 40, 64])
+def test_stedc_after_a_failed_stage(helpers, n):
+    """One subtree is the whole solve: after an error of an earlier stage it leaves its inputs and outputs alone."""
+    d, _, w, z, code = _stedc(helpers, n, n, 3)
+    assert code == 3 and np.array_equal(w, d) and np.all(z == 7.0)

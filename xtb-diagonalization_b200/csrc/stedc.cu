@@ -66,7 +66,6 @@ struct DcBufs {
   int* sperm;     // sorted position -> local column
   int* typ;       // column type by sorted position (1: upper only, 2: both, 3: lower only, 4: deflated)
   int* ndl;       // scratch list of non-deflated positions
-  int* cand;      // pair candidate flags
   int* slotOf;    // survivor index -> GEMM slot
   int* srcCol;    // Qc column -> local source column in Qa
   int* rotI;
@@ -977,11 +976,11 @@ __device__ __forceinline__ void sub_vectors(const SubShared& S, const double (*q
 // on the size, and 16 take twice the rounds.
 // The subtree's tears are those of its ends and of its leaves' ends.  Results go to dd / dnext and the diagonal block of
 // both eigenvector buffers (the entry state of the first level above), or, for the whole matrix (depth 0), straight to
-// d_out (unscaled) and z.
+// d_out (unscaled) and z's first m_cols columns.
 __global__ void __launch_bounds__(kSubThreads, 1) dc_subtree_kernel(int ntot, int depth, const double* d,
                                                                  const double* e, const double* scale_in,
                                                                  double* dd, double* dnext, double* qa, double* qb, int ld,
-                                                                 double* d_out, double* z, int ldz, DeviceStatus* st) {
+                                                                 double* d_out, double* z, int ldz, int m_cols, DeviceStatus* st) {
   extern __shared__ __align__(16) unsigned char sub_smem[];
   SubShared& S = *reinterpret_cast<SubShared*>(sub_smem);
   __shared__ double red[32];
@@ -990,6 +989,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) dc_subtree_kernel(int ntot, in
   tree_block(blockIdx.x, depth, lo, hi);
   const int m = hi - lo;
   if (m <= 0 || m > kSubMax) return;
+  const int failed = ld_volatile_i32(&st->code);  // an earlier stage's; another CTA may record one meanwhile
   double sc;
   if (depth == 0) {  // the whole matrix: its scale is found here
     double x = 0.0;
@@ -1004,7 +1004,9 @@ __global__ void __launch_bounds__(kSubThreads, 1) dc_subtree_kernel(int ntot, in
     (&S.q[1][0][0])[t] = 0.0;
     (&S.u[0][0])[t] = 0.0;
   }
-  __syncthreads();
+  // Columns start in range: a ranking on non-finite input might leave one unwritten.
+  if (tid < kSubMax) S.perm[tid] = S.col[tid] = S.dcol[tid] = S.ri[tid] = S.rj[tid] = S.org[tid] = S.out[tid] = 0;
+  if (__syncthreads_or(failed)) return;
   const int L = tree_depth(m, kSubLeaf);
   for (int i = tid; i < m; i += kSubThreads) {
     S.q[0][i][i] = d[lo + i] * inv;
@@ -1156,7 +1158,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) dc_subtree_kernel(int ntot, in
   if (depth == 0) {
     const double up = sc > 0.0 ? sc : 1.0;
     for (int i = tid; i < m; i += kSubThreads) d_out[i] = S.d[cur][i] * up;
-    for (int t = tid; t < m * m; t += kSubThreads) {
+    for (int t = tid; t < m * m_cols; t += kSubThreads) {
       const int c = t / m, r = t - c * m;
       z[(size_t)r + (size_t)c * ldz] = q[r][c];
     }
@@ -1293,7 +1295,7 @@ size_t stedc_work_bytes(int n) {
   for (int i = 0; i < 4; ++i) add(nn * sizeof(double));  // Qa Qb Qc Up
   for (int i = 0; i < 11; ++i) add(n * sizeof(double));  // rtau sd sz dlam zk zh lam dval rotc rots dnext
   add(sizeof(double) * 4);             // scale
-  for (int i = 0; i < 9; ++i) add(n * sizeof(int));     // sperm typ ndl cand slotOf srcCol rotI rotJ rorg
+  for (int i = 0; i < 8; ++i) add(n * sizeof(int));     // sperm typ ndl slotOf srcCol rotI rotJ rorg
   // per level: posMerge, merges, info, gemm descriptors (levels <= 32)
   add((size_t)32 * n * sizeof(int));
   add((size_t)32 * (n / 2 + 2) * sizeof(MergeDesc));
@@ -1344,7 +1346,6 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
   B.sperm = carve<int>(p, n);
   B.typ = carve<int>(p, n);
   B.ndl = carve<int>(p, n);
-  B.cand = carve<int>(p, n);
   B.slotOf = carve<int>(p, n);
   B.srcCol = carve<int>(p, n);
   B.rotI = carve<int>(p, n);
@@ -1439,7 +1440,7 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
   }
   if (D == 0) {
     dc_subtree_kernel<<<1, kSubThreads, sizeof(SubShared), s>>>(n, 0, d, e, nullptr, nullptr, nullptr, nullptr, nullptr, 0, d,
-                                                                z, ldz, st);
+                                                                z, ldz, m_cols, st);
     note_launches();
     return cudaGetLastError();
   }
@@ -1454,7 +1455,7 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
   }
   if (D > 0) {
     dc_subtree_kernel<<<1 << D, kSubThreads, sizeof(SubShared), s>>>(n, D, d, e, B.scale, B.dd, dnext, B.Qa, B.Qb, n, nullptr,
-                                                                     nullptr, 0, st);
+                                                                     nullptr, 0, 0, st);
     note_launches();
     l_first = std::max(0, L - D);  // levels[l] holds the merges at depth L - 1 - l
   }
