@@ -70,6 +70,7 @@ constexpr int kSytrdTailMax = 128;
 template <typename T>
 cudaError_t sytrd_tail_launch(const SytrdParams<T>& p, int skip_dinit, cudaStream_t s);
 // Variant reading the upper triangle of p.afull == p.aout in place (FP64, rows in shared memory, n <= 2048).
+bool sytrd_upper_inplace_supported(const SytrdPlan& pl);
 cudaError_t sytrd_launch_upper_inplace(const SytrdParams<double>& p, const SytrdPlan& pl, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------------------------- utilities

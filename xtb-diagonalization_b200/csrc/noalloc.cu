@@ -58,7 +58,7 @@ extern "C" int xtb_dsytrd_upper_noalloc(int n, double* a, int lda, double* d, do
   if (err == cudaSuccess) err = scratch_address(&base);
   if (err != cudaSuccess) return -1000 - (int)err;
   const SytrdPlan pl = sytrd_plan<double>(n, sms, (size_t)smem > 2048 ? (size_t)smem - 2048 : (size_t)smem, 0);
-  if (!pl.rows_in_smem) return -4;
+  if (!sytrd_upper_inplace_supported(pl)) return -4;
 
   SytrdParams<double> p{};
   p.n = n;

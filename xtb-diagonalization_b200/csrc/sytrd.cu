@@ -824,15 +824,19 @@ cudaError_t launch_one(const SytrdParams<T>& p, int G, size_t smem, cudaStream_t
   return err;
 }
 
-template <int NT, int CPT, int RR>
-cudaError_t launch_upper_inplace(const SytrdParams<double>& p, int G, size_t smem, cudaStream_t s) {
-  auto kern = sytrd_resident_kernel<double, NT, CPT, RR, true>;
-  cudaError_t err = allow_max_dynamic_smem(kern);
-  if (err != cudaSuccess) return err;
-  void* args[] = {(void*)&p};
-  err = cudaLaunchCooperativeKernel((void*)kern, dim3(G), dim3(NT), args, smem, s);
-  note_launches();
-  return err;
+// The in-place kernel of a plan, or null: every plan of n <= 2048, whose rows per CTA depend on the device's SMs.
+using UpperKernel = void (*)(SytrdParams<double>);
+UpperKernel upper_inplace_kernel(const SytrdPlan& pl) {
+  switch (pl.threads * 1000 + pl.cpt * 10 + pl.reg_rows) {
+    case 128024: return sytrd_resident_kernel<double, 128, 2, 4, true>;
+    case 128028: return sytrd_resident_kernel<double, 128, 2, 8, true>;
+    case 128044: return sytrd_resident_kernel<double, 128, 4, 4, true>;
+    case 128048: return sytrd_resident_kernel<double, 128, 4, 8, true>;
+    case 256044: return sytrd_resident_kernel<double, 256, 4, 4, true>;
+    case 256048: return sytrd_resident_kernel<double, 256, 4, 8, true>;
+    case 256088: return sytrd_resident_kernel<double, 256, 8, 8, true>;
+  }
+  return nullptr;
 }
 
 // Every slot of the ring starts empty (all ones), as far as the launch uses it.
@@ -843,20 +847,21 @@ cudaError_t empty_ring(const SytrdParams<T>& p, cudaStream_t s) {
 
 }  // namespace
 
-// The in-place variant (upper triangle read where it lies; FP64; n <= 2048).
+// The in-place variant (upper triangle read where it lies; rows on chip; FP64; n <= 2048).
+bool sytrd_upper_inplace_supported(const SytrdPlan& pl) { return pl.rows_in_smem && upper_inplace_kernel(pl) != nullptr; }
+
 cudaError_t sytrd_launch_upper_inplace(const SytrdParams<double>& p, const SytrdPlan& pl, cudaStream_t s) {
   if (p.n <= 0) return cudaSuccess;
-  if (!pl.rows_in_smem) return cudaErrorInvalidValue;
+  if (!sytrd_upper_inplace_supported(pl)) return cudaErrorInvalidValue;
   cudaError_t err = empty_ring(p, s);
   if (err != cudaSuccess) return err;
-  switch (pl.threads * 1000 + pl.cpt * 10 + pl.reg_rows) {
-    case 128024: return launch_upper_inplace<128, 2, 4>(p, pl.grid, pl.smem, s);
-    case 128044: return launch_upper_inplace<128, 4, 4>(p, pl.grid, pl.smem, s);
-    case 256044: return launch_upper_inplace<256, 4, 4>(p, pl.grid, pl.smem, s);
-    case 256048: return launch_upper_inplace<256, 4, 8>(p, pl.grid, pl.smem, s);
-    case 256088: return launch_upper_inplace<256, 8, 8>(p, pl.grid, pl.smem, s);
-  }
-  return cudaErrorInvalidValue;
+  const UpperKernel kern = upper_inplace_kernel(pl);
+  err = allow_max_dynamic_smem(kern);
+  if (err != cudaSuccess) return err;
+  void* args[] = {(void*)&p};
+  err = cudaLaunchCooperativeKernel((void*)kern, dim3(pl.grid), dim3(pl.threads), args, pl.smem, s);
+  note_launches();
+  return err;
 }
 
 template <typename T>
