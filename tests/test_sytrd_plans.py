@@ -1,7 +1,7 @@
 """The plans of the resident reduction for devices with fewer SMs (a partition of a GPU), on the CPU: the library's own
 planning functions are called through their exported names.
 
-The no-allocation entry takes every n up to 1792 whose rows the device holds on chip.  Rows per CTA, and with them the
+Option "sytrd_grid" takes any number of CTAs, however many rows each then owns.  The no-allocation entry takes every n up to 1792 whose rows the device holds on chip.  Rows per CTA, and with them the
 kernel a plan selects, depend on the number of SMs.
 """
 import ctypes
@@ -43,3 +43,13 @@ def test_every_plan_on_chip_has_a_kernel(functions, sms):
             assert pl.rows_in_smem, (n, sms)
         if pl.rows_in_smem:
             assert pl.supported and supported(ctypes.byref(pl)), (n, sms)
+
+
+@pytest.mark.parametrize("n", [1, 63, 500, 1788, 2049, 4096, 4097, 8192, 8193, 16384])
+def test_a_chosen_grid_fits_in_shared_memory(functions, n):
+    plan, _ = functions
+    for grid in range(1, 149):
+        pl = plan(n, 148, MAX_SMEM, grid)
+        assert pl.supported and pl.smem <= MAX_SMEM and grid <= pl.grid <= 148, grid
+        if n <= 1024 or grid >= 64:
+            assert pl.grid == grid

@@ -880,8 +880,7 @@ template <typename T>
 SytrdPlan sytrd_plan(int n, int num_sms, size_t max_smem, int grid_override) {
   SytrdPlan pl{};
   // Small problems: fewer CTAs, at least ~4 rows each.
-  const int G = grid_override > 0 ? grid_override : max(1, min(num_sms, (n + 3) / 4));
-  pl.grid = G;
+  pl.grid = grid_override > 0 ? grid_override : max(1, min(num_sms, (n + 3) / 4));
   // Few warps keep the block syncs and cross-warp sums short; at least four, one per scheduler.
   if (n <= 256) { pl.threads = 128; pl.cpt = 2; }
   else if (n <= 512) { pl.threads = 128; pl.cpt = 4; }
@@ -891,7 +890,12 @@ SytrdPlan sytrd_plan(int n, int num_sms, size_t max_smem, int grid_override) {
   else { pl.threads = 1024; pl.cpt = n <= 8192 ? 8 : 16; }
   // Registers hold the rows of a CTA that has few of them; blocks of more than 256 threads have none to spare.
   constexpr int BL = sytrd_row_block<T>();
-  pl.rows_per_cta = BL * (((n + BL - 1) / BL + G - 1) / G);
+  // A chosen grid so small that even the sums of a CTA's rows outgrow its shared memory is raised to one that works: the
+  // results are the same for every grid.
+  for (;; ++pl.grid) {
+    pl.rows_per_cta = BL * (((n + BL - 1) / BL + pl.grid - 1) / pl.grid);
+    if (pl.grid >= num_sms || sytrd_smem_bytes<T>(n, pl.rows_per_cta, pl.threads, pl.cpt, 0, nullptr) <= max_smem) break;
+  }
   const int reg_rows = pl.reg_rows = pl.threads > 256 ? 0 : pl.rows_per_cta <= 4 ? 4 : 8;
   const int others = max(0, pl.rows_per_cta - reg_rows);
   const size_t with_rows = sytrd_smem_bytes<T>(n, pl.rows_per_cta, pl.threads, pl.cpt, others, &pl.ldr);
