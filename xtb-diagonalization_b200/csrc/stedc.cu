@@ -972,8 +972,8 @@ __device__ __forceinline__ void sub_vectors(const SubShared& S, const double (*q
 // then the product with the blocks' vectors in register tiles.  The steps and tests are those of the level kernels below.
 // What bounds it is latency: a few hundred dependent operations per level, in place of nine launches.  It took the place
 // of Jacobi leaves of 16 and the level kernels up to 64: the whole tridiagonal solve 203 -> 59 us at n = 37, 346 -> 193 at
-// 130, 548 -> 344 at 412 (with the branch-free divisions).  Leaves of 8 because a Jacobi round's latency does not depend
-// on the size, and 16 take twice the rounds.
+// 130, 548 -> 344 at 412 (with the branch-free divisions; now 59, 177 and 289).  Leaves of 8 because a Jacobi round's
+// latency does not depend on the size, and 16 take twice the rounds.
 // The subtree's tears are those of its ends and of its leaves' ends.  Results go to dd / dnext and the diagonal block of
 // both eigenvector buffers (the entry state of the first level above), or, for the whole matrix (depth 0), straight to
 // d_out (unscaled) and z's first m_cols columns.

@@ -41,10 +41,10 @@
 // The ring has three thirds of H slots; step t uses slot t mod 3H.  In step t = bH + 1, after publishing, the owner
 // of a row puts the empty pattern back into its entries of third (b - 1) mod 3 and every thread executes a fence.
 // Every CTA has then read all of third (b - 1) mod 3: a CTA reads step s only if it has a row in step s + 1, which it
-// publishes after reading, and this CTA has read every pair of step t - 1 = bH.  The third is polled again from step (b + 2)H on; by then the reader has seen
-// a later publish of the same owner thread (step bH + 2 or later, H >= 2) and executed its own fence of step
-// (b + 1)H + 1, so the emptying happens before the poll.  A fence costs about 1000 cycles while stores are in flight,
-// so a third has 32 slots (8: 2 % slower).
+// publishes after reading, and this CTA has read every pair of step t - 1 = bH.  The third is polled again from step
+// (b + 2)H on; by then the reader has seen a later publish of the same owner thread (step bH + 2 or later, H >= 2) and
+// executed its own fence of step (b + 1)H + 1, so the emptying happens before the poll.  A fence costs about 1000 cycles
+// while stores are in flight, so a third has 32 slots (8: 2 % slower).
 #include <type_traits>
 
 #include "common.cuh"

@@ -25,10 +25,9 @@ __host__ __device__ inline int gram_slices(int rows, int S) { return max(1, min(
 // G's strict upper triangle is kept transposed in the strict lower triangle of the same array.  M = G12 T2 goes where T12
 // will be; -T1 M goes where G12 was (nothing reads it again) and is then copied over M.  Both products run on 8 x 8 tiles
 // of the FP64 tensor pipe (an FP32 block too: its entries are widened, so its sums only gain), a warp per tile.  The
-// recurrence is sequential only inside the diagonal blocks.  What bounds it: the latency of the chain of joins on one SM;
-// a kernel that
-// formed T12's rows one after another and divided for every index took 159 us for 14 blocks of 128 (two blocks: 115),
-// now 50 (22).
+// recurrence is sequential only inside the diagonal blocks.  What bounds it: the latency of the chain of joins on one SM; a
+// kernel that formed T12's rows one after another and divided for every index took 159 us for 14 blocks of 128 (two
+// blocks: 115), now 50 (22).
 // The leading dimension nb + kWyPad puts the 4 x 8 elements of a tile's operand on different banks.
 constexpr int kWyThreads = 512;
 
