@@ -1,6 +1,7 @@
 // Kernels that call single device helpers of the library, and calls of its internal stages, for
 // tests/test_gpu_device_helpers.py.
 #include "common.cuh"
+#include "gemm.cuh"
 #include "kernels.h"
 
 using namespace xtbeig;
@@ -46,6 +47,28 @@ __global__ void divide_kernel(int n, const double* a, const double* x, double* r
 extern "C" int run_divide(int n, const double* a, const double* x, double* rcp, double* quot, double* plain) {
   divide_kernel<<<(n + 255) / 256, 256>>>(n, a, x, rcp, quot, plain);
   return (int)cudaDeviceSynchronize();
+}
+
+// A launch that the runtime refuses on the host (on the legacy stream while another stream captures): what the grouped
+// GEMM's launcher returns.  The descriptors are empty problems, so a launch that went through would do nothing.
+extern "C" int run_refused_gemm(int nprob) {
+  cudaStream_t s = nullptr;
+  cudaGraph_t graph = nullptr;
+  GemmDesc<double>* empty = nullptr;
+  const size_t bytes = (nprob + 1) * sizeof(*empty);
+  cudaError_t err = cudaMalloc(&empty, bytes);
+  if (err == cudaSuccess) err = cudaMemset(empty, 0, bytes);
+  if (err == cudaSuccess) err = cudaDeviceSynchronize();
+  if (err == cudaSuccess) err = cudaStreamCreate(&s);
+  if (err == cudaSuccess) err = cudaStreamBeginCapture(s, cudaStreamCaptureModeGlobal);
+  if (err != cudaSuccess) return -1;
+  const int refused = (int)gemm_grouped_launch<double>(empty, nprob, 1, 64, nullptr);
+  cudaStreamEndCapture(s, &graph);
+  if (graph) cudaGraphDestroy(graph);
+  cudaStreamDestroy(s);
+  cudaGetLastError();
+  cudaFree(empty);
+  return refused;
 }
 
 // The divide and conquer stage on device buffers d (n), e (n - 1), z (ldz x n), with a status word that starts at `code`.

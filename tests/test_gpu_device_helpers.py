@@ -66,6 +66,12 @@ def test_branch_free_division(helpers, case):
     assert np.abs(quot.view(np.int64) - plain.view(np.int64)).max() <= 1
 
 
+def test_refused_gemm_launch_is_reported(helpers):
+    """The launcher's own result is the only report of a launch that the runtime refuses: cudaErrorStreamCaptureImplicit."""
+    assert helpers.run_refused_gemm(0) == 0  # nothing to launch
+    assert helpers.run_refused_gemm(1) == 906
+
+
 def _stedc(helpers, n, m_cols, code):
     import torch
 

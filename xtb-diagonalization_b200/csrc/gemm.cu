@@ -82,15 +82,15 @@ cudaError_t gemm_launch(const Src& src, int tiles, cudaStream_t s) {
 }  // namespace
 
 template <typename T>
-void gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, int edge, cudaStream_t s) {
-  if (nprob <= 0 || total_tiles <= 0) return;
+cudaError_t gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, int edge, cudaStream_t s) {
+  if (nprob <= 0 || total_tiles <= 0) return cudaSuccess;
   DescFromMemory<T> src{d_descs, nprob};
-  if (edge == 32) gemm_launch<T, DescFromMemory<T>, 32>(src, total_tiles, s);
-  else gemm_launch<T, DescFromMemory<T>, 64>(src, total_tiles, s);
+  return edge == 32 ? gemm_launch<T, DescFromMemory<T>, 32>(src, total_tiles, s)
+                    : gemm_launch<T, DescFromMemory<T>, 64>(src, total_tiles, s);
 }
 
-template void gemm_grouped_launch<double>(const GemmDesc<double>*, int, int, int, cudaStream_t);
-template void gemm_grouped_launch<float>(const GemmDesc<float>*, int, int, int, cudaStream_t);
+template cudaError_t gemm_grouped_launch<double>(const GemmDesc<double>*, int, int, int, cudaStream_t);
+template cudaError_t gemm_grouped_launch<float>(const GemmDesc<float>*, int, int, int, cudaStream_t);
 
 template <typename T>
 GemmDesc<T> gemm_problem(int M, int N, int K, T alpha, const T* A, int lda, int transA, const T* B, int ldb,
@@ -137,8 +137,7 @@ cudaError_t gemm_group(DescArena& arena, const GemmDesc<T>* probs, int nprob, cu
   }
   cudaError_t err = cudaMemcpyAsync(d, h, (size_t)nprob * sizeof(GemmDesc<T>), cudaMemcpyHostToDevice, s);
   if (err != cudaSuccess) return err;
-  gemm_grouped_launch<T>(reinterpret_cast<GemmDesc<T>*>(d), nprob, tb, edge, s);
-  return cudaGetLastError();
+  return gemm_grouped_launch<T>(reinterpret_cast<GemmDesc<T>*>(d), nprob, tb, edge, s);
 }
 
 cudaError_t gemm_run(DescArena& arena, const TcGemm& tc, const GemmDesc<double>* probs, int nprob, cudaStream_t s) {

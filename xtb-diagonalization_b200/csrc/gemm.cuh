@@ -63,8 +63,8 @@ int gemm_tile_edge(long tiles64, long tiles32) {
 }
 
 // Launch a group: descs (device) holds nprob descriptors whose tiles_m, tiles_n count tiles of `edge` and whose
-// tile_begin are their prefix sum; total_tiles their sum.
+// tile_begin are their prefix sum; total_tiles their sum.  Returns the launch's error, which no later call reports.
 template <typename T>
-void gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, int edge, cudaStream_t s);
+cudaError_t gemm_grouped_launch(const GemmDesc<T>* d_descs, int nprob, int total_tiles, int edge, cudaStream_t s);
 
 }  // namespace xtbeig

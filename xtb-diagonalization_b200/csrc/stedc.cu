@@ -1488,7 +1488,8 @@ cudaError_t stedc_device(int n, double* d, double* e, double* z, int ldz, void* 
     if (partial) {
       dc_partial_kernel<<<1, 1024, 0, s>>>(B, m_cols); note_launches();
     }
-    gemm_grouped_launch<double>(B.gdesc, 2 * nm, tiles[l], edges[l], s);
+    err = gemm_grouped_launch<double>(B.gdesc, 2 * nm, tiles[l], edges[l], s);
+    if (err != cudaSuccess) return err;
     dc_place_kernel<<<dim3(nm, std::min(maxn, 65535)), 256, 0, s>>>(B, dnext, partial ? m_cols : n);
     note_launches();
     err = cudaGetLastError();
