@@ -1,8 +1,9 @@
 """The plans of the resident reduction for devices with fewer SMs (a partition of a GPU), on the CPU: the library's own
 planning functions are called through their exported names.
 
-Option "sytrd_grid" takes any number of CTAs, however many rows each then owns.  The no-allocation entry takes every n up to 1792 whose rows the device holds on chip.  Rows per CTA, and with them the
-kernel a plan selects, depend on the number of SMs.
+Option "sytrd_grid" takes any number of CTAs, however many rows each then owns.  The no-allocation entry takes every n up
+to 1792 whose rows the device holds on chip.  Rows per CTA, and with them the kernel a plan selects, depend on the number
+of SMs.
 """
 import ctypes
 import re

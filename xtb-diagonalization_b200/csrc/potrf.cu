@@ -187,7 +187,7 @@ __device__ __forceinline__ void leaf_follow_steps(double (&m)[16][2], int b, con
 // -U(k, i) W(k, k)), so the inverse costs no further step.  The owner warp runs down its 16 rows by shuffles alone,
 // leaving each final row in shared memory; the warps below follow it at their own pace (a row counter, no block
 // barrier).  One block alone (with its panel update): about 40 k cycles, where panels of 8 columns with block barriers and
-// a separate block-wise inverse took 57 k; potrf + inverse n = 130 152 -> 122 us, 619 493 -> 407, 1788 1.40 -> 1.05 ms (of
+// a separate block-wise inverse took 57 k; potrf + inverse n = 130 149 -> 120 us, 619 493 -> 407, 1788 1.42 -> 1.07 ms (of
 // which the tiles of the trailing update, gemm_tile, gave a part).
 // With a panel (the kp x nb block row U(j0 - kp : j0, j0 : j0 + nb), ld lda), the block's trailing update
 // A -= P^T P runs first, by matrix instructions (gsm: the tile pipeline's region, free while the leaf runs, holds P).

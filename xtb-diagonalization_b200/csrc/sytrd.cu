@@ -659,7 +659,7 @@ __device__ __forceinline__ void warp_row_sums_strided(float (&acc)[ROWS], float*
 // the others pass over their rows (a dependent chain of a sum, a reciprocal square root and a division).
 // A warp's own copy of (v, w) in shared memory gives it the values at its rows.  Bound by latency: the pass and its
 // reduce-scatter, one sync, a warp sum by matrix instruction.  It replaced a kernel that kept the block in shared memory
-// with four block syncs and two shuffled sums per column (2.0 us per column of a block of 64, now 0.7: 130 -> 45 us).
+// with four block syncs and two shuffled sums per column (2.0 us per column of a block of 64, now 0.6: 130 -> 40 us).
 template <typename T, int M>
 __global__ void __launch_bounds__(2 * M + (M == 64 ? 32 : 0), 1) sytrd_tail_kernel(SytrdParams<T> p, int skip_dinit) {
   constexpr int NW = M / 16, CJ = M / 32;
