@@ -398,8 +398,9 @@ void stage_sytrd(Call& k, int n, const T* dfull, int ldf, T* dout, int lda, T* d
   }
   if (tail > 1) {
     p.k_stop = tail - 1;
-    p.hand = k.template dev<T>("sytrd.hand", (size_t)tail * tail);
+    p.hand = k.template dev<T>("sytrd.hand", (size_t)tail * tail + 1);
     p.ldh = tail;
+    p.floor2 = p.hand + (size_t)tail * tail;
     if (!k.ok()) return;
   }
   k.check(sytrd_launch<T>(p, pl, k.s), "sytrd launch");

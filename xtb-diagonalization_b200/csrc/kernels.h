@@ -43,6 +43,7 @@ struct SytrdParams {
   int k_stop;
   T* hand;
   int ldh;
+  T* floor2;  // with k_stop: the hand-over of ColumnFloor's bound from the grid kernel to the tail
 };
 
 struct SytrdPlan {

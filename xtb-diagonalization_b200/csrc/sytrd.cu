@@ -90,6 +90,28 @@ struct __align__(2 * sizeof(T)) Pair {
   T a, b;
 };
 
+// A column of the trailing block whose squared norm is below a bound is taken as zero (tau = 0; its elements, but not alpha,
+// are dropped).  Where a block vanishes, as in a matrix of low rank, rounding leaves u |A|, u^2 |A|, ... of it column by
+// column, until the squares underflow: with a norm good to a few bits v and tau no longer fit together and Q was not
+// orthogonal (ones(33): |Q^T Q - I| = 0.13).  The bound is where the sum of n <= 2^14 squares loses its last bits to
+// underflow, but never more than 2^-10 u of the largest column so far, so that a matrix that is small itself keeps its
+// columns: what is dropped lies below the rounding of the reduction.
+template <typename T>
+struct ColumnFloor;
+template <>
+struct ColumnFloor<double> {
+  static constexpr double kTiny = 0x1p-1000, kOfLargest = 0x1p-126;
+};
+template <>
+struct ColumnFloor<float> {
+  static constexpr float kTiny = 0x1p-110f, kOfLargest = 0x1p-68f;
+};
+// The bound after a column of squared norm s2.
+template <typename T>
+__device__ __forceinline__ T next_floor2(T floor2, T s2) {
+  return fmax(floor2, fmin(ColumnFloor<T>::kTiny, s2 * ColumnFloor<T>::kOfLargest));
+}
+
 // Sum of N values (N a power of two) read from shared memory, as a balanced tree: log2 N dependent additions.
 template <int N, typename T>
 __device__ __forceinline__ T tree_sum(const T* p, int stride) {
@@ -258,10 +280,10 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
   T* red = reinterpret_cast<T*>(vy + R + 8);                 // [NW][R + 8]
   T* colk = red + (size_t)(R + 8) * NW;                      // [8]
   T* bred = colk + 8;                                        // [2][NW]
-  T* scal = bred + 2 * NW;                                   // [4]
+  T* scal = bred + 2 * NW;                                   // [4], and the column floor before an even and an odd column
   T* rows = nullptr;
   if constexpr (kSmemRows) {
-    const size_t off = (size_t)(reinterpret_cast<unsigned char*>(scal + 4) - smem_raw);
+    const size_t off = (size_t)(reinterpret_cast<unsigned char*>(scal + 6) - smem_raw);
     rows = reinterpret_cast<T*>(smem_raw + ((off + 15) & ~size_t(15)));
   } else {
     rows = p.grows + (size_t)cta * R * ldr;
@@ -302,6 +324,7 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
     vk[i] = wk[i] = T(0);
   }
   for (int q = tid; q < R + 8; q += NT) vy[q] = Pair<T>{T(0), T(0)};
+  if (tid < 2) scal[4 + tid] = T(0);
   if (cta == 0 && tid == 0 && n >= 1) {
     T dn = load(n - 1, n - 1);
     p.d[n - 1] = dn;
@@ -431,14 +454,13 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
       }
       // ---- 4. Householder vector (identical in every CTA: same data, same order).
       const T xn2 = tree_sum<NW>(bred, 1);
-      const T alpha = scal[0];
+      const T alpha = scal[0], s2 = alpha * alpha + xn2, floor2 = scal[4 + (k & 1)];
       T beta, tau, scale;
-      if (xn2 == T(0)) {
+      if (xn2 == T(0) || s2 < floor2) {
         beta = alpha; tau = T(0); scale = T(0);
       } else {
         // beta = -sign(alpha) ||(alpha, x)||, tau = (beta - alpha)/beta = 1 + |alpha|/||.||: one reciprocal square
         // root and one division.
-        const T s2 = alpha * alpha + xn2;
         const T rn = rsqrt(s2);
         const T nrm = s2 * rn;
         beta = alpha >= T(0) ? -nrm : nrm;
@@ -466,7 +488,10 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
       };
       if (tid < nq) keep_row(tid, my_row, ax_own, col_own);
       for (int q = tid + NT; q < nq; q += NT) keep_row(q, row_of(q), red[q], rows[(size_t)(q - RR) * ldr + (k - 1)]);
-      if (cta == 0 && tid == NT - 1) { p.e[k - 1] = beta; p.tau[k - 1] = tau; }
+      if (tid == NT - 1) {
+        scal[4 + ((k - 1) & 1)] = next_floor2(floor2, s2);
+        if (cta == 0) { p.e[k - 1] = beta; p.tau[k - 1] = tau; }
+      }
       if (phase == 1) {  // empty the third that every CTA has finished reading (see above)
         if (!first_block) {
           T* base = p.xch + (size_t)third * H * slot_ld;
@@ -583,6 +608,7 @@ __global__ void __launch_bounds__(NT, 1) sytrd_resident_kernel(SytrdParams<T> p)
   // the last exchange, so every row of the block is complete.
   if (p.k_stop > 0 && k_end <= n - 1) {
     const int m = p.k_stop + 1;
+    if (cta == 0 && tid == 0) *p.floor2 = scal[4 + ((k_end - 1) & 1)];
     auto hand_row = [&](int q, auto get) {
       const int r = row_of(q);
       const Pair<T> o = vy[q];
@@ -690,6 +716,7 @@ __global__ void __launch_bounds__(2 * M + (M == 64 ? 32 : 0), 1) sytrd_tail_kern
     p.d[m - 1] = dn;
     p.aout[(size_t)(m - 1) + (size_t)(m - 1) * p.lda] = dn;
   }
+  T floor2 = skip_dinit ? *p.floor2 : T(0);
   __syncwarp();
   for (int k = m - 1; k >= 1; --k) {
     // One column over the first J column groups and ROWS rows per warp (the others lie beyond k).
@@ -708,11 +735,12 @@ __global__ void __launch_bounds__(2 * M + (M == 64 ? 32 : 0), 1) sytrd_tail_kern
           part = fma(xs[j], xs[j], part);
           if (j == jk) alpha = __shfl_sync(0xffffffffu, x[j], lk);
         }
-        const T xn2 = warp_sum_mma(part);
-        if (xn2 == T(0)) {
+        const T xn2 = warp_sum_mma(part), s2 = alpha * alpha + xn2;
+        const bool none = xn2 == T(0) || s2 < floor2;
+        floor2 = next_floor2(floor2, s2);
+        if (none) {
           beta = alpha; tau = T(0); scale = T(0);
         } else {
-          const T s2 = alpha * alpha + xn2;
           const T rn = rsqrt(s2);
           const T nrm = s2 * rn;
           beta = alpha >= T(0) ? -nrm : nrm;
@@ -869,7 +897,7 @@ size_t sytrd_smem_bytes(int n, int R, int NT, int cpt, int smem_rows, int* ldr_o
   const int align = 16 / (int)sizeof(T);
   const int ldr = ((n + align - 1) / align) * align;
   const int NW = NT / 32;
-  const size_t elems = (size_t)NT * cpt + 2 * ((size_t)R + 8) + ((size_t)R + 8) * NW + 8 + 2 * (size_t)NW + 4;
+  const size_t elems = (size_t)NT * cpt + 2 * ((size_t)R + 8) + ((size_t)R + 8) * NW + 8 + 2 * (size_t)NW + 6;
   size_t bytes = (elems * sizeof(T) + 15) & ~size_t(15);
   bytes += (size_t)smem_rows * ldr * sizeof(T);
   if (ldr_out) *ldr_out = ldr;
